@@ -6,8 +6,6 @@
 // scales [num_blocks, Hkv] fp32 (value = stored * scale).
 #include <cuda_fp8.h>
 
-#include <cstdlib>
-
 #include "common.cuh"
 #include "host.h"
 
@@ -110,303 +108,416 @@ __global__ void kv_gather_kernel(const void* __restrict__ k_cache, const void* _
 }
 
 // ---------------------------------------------------------------------------------------------
-// Paged decode attention: one query token per sequence.  Grid (B, Hkv * head groups, nsplit); a CTA streams
-// its partition of the sequence's pages, scores the query heads of its kv head, and keeps an online softmax.
-// nsplit == 1 writes the output directly; otherwise unnormalised partials + (max, sum) go to a workspace for
-// the merge kernel.
+// Paged decode attention: one query token per sequence.  Grid (B, Hkv, parts of the context).
+//
+// Bound by the bytes of the cache.  With scalar FMAs it was not: every cache row cost G dot products, their shuffles over the
+// lanes of the row and (fp8) a conversion per byte in every head group, 86 us for 98 MB of fp8 cache with four query
+// heads per kv head (32 sequences of ~1500 tokens, 8 kv heads), and a single sequence kept 8 CTAs busy (25 us at 1024
+// tokens).  Here both products run on the tensor cores (mma.m16n8k16: the query heads of one kv head are too few rows for
+// a tcgen05 tile) and the parts of a context that a cluster of CTAs works through are merged over distributed shared
+// memory, so the split needs neither a plan on the host nor a workspace nor a second kernel.
+//
+// A warp takes pages (16 tokens) in turn; its K and V rows arrive in a ring of its own by 16-byte cp.async copies.
+//   scores:  A = the query heads, one per row (rows r and r + GP hold the same head), B = the page's keys.
+//   output:  A = the probabilities, B = the page's values.  Probabilities keep 24 bits: p = hi + mid + lo in the 16-bit type,
+//            and rows r, r + GP, r + 2 GP of A are those three parts of the same head, so the split costs no product of its
+//            own up to four heads (GP = 8: a second one).  The rows of a head are added up once, at the end.
+// Contraction indices may be permuted freely, so both operands are read from shared memory 16 bytes per lane: lane
+// (r = lane / 4, c = lane % 4) owns the dims of chunks c, c + 4, .. of key r, and dims 16 r .. 16 r + 15 of the values of
+// tokens 2 c, 2 c + 1, 2 c + 8, 2 c + 9.  The chunk swizzle below makes both patterns free of bank conflicts.
+// fp8 rows become fp16 (exact).  The page's key scale multiplies the score; its value scale, less its largest exponent
+// so far (a power of two, divided out at the end), the probability, which carries a factor 2^14 to stay clear of
+// fp16's subnormals.  Queries of fp8 caches are scaled by a power of two per head to lie in [2^13, 2^14) at most.
 // ---------------------------------------------------------------------------------------------
-constexpr int DEC_THREADS = 128;
 constexpr int DEC_CHUNK = 64;   // partitions are multiples of this many tokens
 constexpr int DEC_MAX_G = 8;
-constexpr int DEC_UNROLL = 4;   // cache rows in flight per lane group
-constexpr int DEC_DEFAULT_MODE = 3;   // row loop of the decode kernel when B200FW_DECODE_MODE is unset
+constexpr int DEC_MAX_CLUSTER = 8;
 constexpr float DEC_LOG2E = 1.4426950408889634f;
 constexpr float DEC_LN2 = 0.6931471805599453f;
 
 template <bool FP8>
-__device__ __forceinline__ void dec_unpack(const uint4& u, float* f);
-template <>
-__device__ __forceinline__ void dec_unpack<false>(const uint4& u, float* f) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 t = unpack_bf16x2(w[j]);
-    f[2 * j] = t.x;
-    f[2 * j + 1] = t.y;
+struct DecCfg {
+  static constexpr int ROW = HD * (FP8 ? 1 : 2);      // bytes of a cache row
+  static constexpr int CPR = ROW / 16;                // 16-byte chunks per row
+  static constexpr int TILE = PAGE * ROW;             // one page of K or V
+  static constexpr int STAGES = FP8 ? 4 : 3;
+  static constexpr int RING = STAGES * 2 * TILE;      // per warp
+  // chunk of row t is stored at chunk ^ swz(t): keys of two neighbouring tokens differ in bit 2, values of four tokens
+  // two apart differ in the two bits that the two chunks of a quarter warp leave free
+  static __device__ __forceinline__ int swz(int t) {
+    const int b2 = ((t >> 2) ^ t) & 1, b1 = (t >> 1) & 1;
+    return (b2 << 2) | (FP8 ? b1 << 1 : b1);
   }
+};
+
+template <bool FP8>
+__device__ __forceinline__ void dec_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if (FP8)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-template <>
-__device__ __forceinline__ void dec_unpack<true>(const uint4& u, float* f) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+// two floats in the operand type (first one in the low half), and back
+template <bool FP8>
+__device__ __forceinline__ uint32_t dec_pack(float x, float y) {
+  if (!FP8) return pack_bf16x2(x, y);
+  const __half2 h = __floats2half2_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <bool FP8>
+__device__ __forceinline__ float2 dec_unpack(uint32_t u) {
+  if (!FP8) return unpack_bf16x2(u);
+  return __half22float2(*reinterpret_cast<const __half2*>(&u));
+}
+// Part `part` of the pair (x, y): 0 the rounded value, 1 what rounding left, 2 what is left after both; none beyond.
+template <bool FP8>
+__device__ __forceinline__ uint32_t dec_part(float x, float y, int part) {
+  uint32_t u = dec_pack<FP8>(x, y);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const __half2_raw r = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>((w[j] >> (16 * h)) & 0xFFFFu),
-                                                       __NV_E4M3);
-      const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&r));
-      f[4 * j + 2 * h] = t.x;
-      f[4 * j + 2 * h + 1] = t.y;
+  for (int i = 0; i < 2; ++i) {
+    if (part > i) {
+      const float2 f = dec_unpack<FP8>(u);
+      x -= f.x;
+      y -= f.y;
+      u = dec_pack<FP8>(x, y);
     }
   }
+  return part > 2 ? 0u : u;
+}
+// two e4m3 bytes (the low half of w) as two halves
+__device__ __forceinline__ uint32_t dec_fp8x2(uint32_t w) {
+  const __half2_raw r = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w & 0xFFFFu), __NV_E4M3);
+  return static_cast<uint32_t>(r.x) | (static_cast<uint32_t>(r.y) << 16);
+}
+__device__ __forceinline__ uint4 dec_lds(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float dec_ld_cluster(uint32_t addr, uint32_t rank) {
+  uint32_t remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  return v;
+}
+__device__ __forceinline__ void dec_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Decode attention over the paged cache, one CTA per (sequence, kv head, head group, partition).
-// A cache row (128 dims) is spread over LPT = 16 (bf16) or 8 (fp8) lanes of a warp, 16 bytes each, so one
-// warp-wide access covers 2 (4) tokens and every lane handles DEC_UNROLL K and V pieces per step; no data is
-// ever shared between lanes through memory.  Each lane group runs its own online softmax over the tokens it sees (running
-// maximum, sum and DPL accumulator dims per head, base-2 exponent domain); groups and warps are merged
-// once at the end with the exact log-sum-exp rule.  GH query heads of the kv head are handled per CTA
-// (their q pieces sit in registers); larger GQA ratios use several CTAs (head groups) per kv head.
-// MODE 0: plain row loop, the K and V pieces of a step are loaded into registers and consumed.
-// MODE 3: every warp owns a ring of three stages in shared memory, filled by 16-byte asynchronous copies
-// (cp.async.cg, no register staging); a lane reads back exactly the bytes it copied, so no barrier is needed, and
-// two steps' worth of K and V rows stay in flight per warp without growing the register count.  (Measured at
-// 256 x 1024: 0.194 ms against 0.231 ms for MODE 0; a four-stage ring, 0.203 ms, and a register software pipeline,
-// 0.283 ms, were tried and dropped.)
-template <bool FP8, int GH, int MODE>
-__global__ void __launch_bounds__(DEC_THREADS) paged_decode_kernel(
+// GP: query heads per kv head, rounded up to a power of two.  clustered: the CTAs along z are one cluster and share a context;
+// otherwise CTA z takes tokens [z * partition, (z + 1) * partition) and, with several, writes its partial result.
+template <bool FP8, int GP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
     const __nv_bfloat16* __restrict__ q, const void* __restrict__ k_cache, const void* __restrict__ v_cache,
     const float* __restrict__ k_scale, const float* __restrict__ v_scale,
     const int* __restrict__ block_tables, const int* __restrict__ context_lens, int max_blocks,
     __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, int Hq, int Hkv,
-    int partition, float scale) {
-  constexpr int ESZ = FP8 ? 1 : 2;
-  constexpr int LPT = HD * ESZ / 16;   // lanes per token row
-  constexpr int TPW = 32 / LPT;        // token rows per warp-wide load
-  constexpr int DPL = 16 / ESZ;        // dims per lane
-  constexpr int U = DEC_UNROLL;
-  static_assert(MODE == 0 || MODE == 3, "row loop: 0 (registers) or 3 (three-stage cp.async ring)");
-  constexpr int STAGES = MODE >= 2 ? MODE : 1;
-  __shared__ float sAcc[DEC_THREADS / 32][GH][HD];
-  __shared__ float sM[DEC_THREADS / 32][GH], sL[DEC_THREADS / 32][GH];
-  extern __shared__ __align__(16) uint8_t dec_ring[];   // [warp][stage][u][K | V][32 lanes x 16 B] (MODE >= 2)
-
+    int partition, float scale, int clustered) {
+  using Cfg = DecCfg<FP8>;
+  extern __shared__ __align__(128) uint8_t dec_ring[];   // [warp][stage][K | V][16 rows]
+  __shared__ float sO[GP][HD], sM[GP], sL[GP];
   const int G = Hq / Hkv;
-  const int groups_per_kv = G / GH;
-  const int b = blockIdx.x, kvh = blockIdx.y / groups_per_kv, hg = blockIdx.y % groups_per_kv;
-  const int split = blockIdx.z, nsplit = gridDim.z;
-  const int head0 = kvh * G + hg * GH;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int group = lane / LPT, sub = lane % LPT;
-  const int ctx = context_lens[b];
-  const int t_begin = split * partition;
-  const int t_end = min(ctx, t_begin + partition);
+  const int b = blockIdx.x, kvh = blockIdx.y, z = blockIdx.z, nz = gridDim.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
+  // The query, the first page numbers (a context that is not split starts at page 0) and the context's length are requested
+  // together: one after the other their latencies are most of what a short context takes.
   const int* table = block_tables + static_cast<size_t>(b) * max_blocks;
-  const size_t tok_stride = static_cast<size_t>(Hkv) * HD * ESZ;
-  const uint8_t* kc = reinterpret_cast<const uint8_t*>(k_cache) + static_cast<size_t>(kvh) * HD * ESZ + sub * 16;
-  const uint8_t* vc = reinterpret_cast<const uint8_t*>(v_cache) + static_cast<size_t>(kvh) * HD * ESZ + sub * 16;
-
-  float qr[GH][DPL], acc[GH][DPL], m[GH], l[GH];
-  const float qs = scale * DEC_LOG2E;
-#pragma unroll
-  for (int g = 0; g < GH; ++g) {
-    const __nv_bfloat16* qp = q + (static_cast<size_t>(b) * Hq + head0 + g) * HD + sub * DPL;
-#pragma unroll
-    for (int d = 0; d < DPL; ++d) {
-      qr[g][d] = __bfloat162float(qp[d]) * qs;
-      acc[g][d] = 0.f;
-    }
-    m[g] = -INFINITY;
-    l[g] = 0.f;
-  }
-
-  // One step of a lane group: U cache rows (their K and V pieces, the block's scales, validity).
-  struct Rows {
-    uint4 kq[U], vq[U];
-    float ks[U], vs[U];
-    bool valid[U];
-  };
-  auto load_rows = [&](Rows& r, int base) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int tok = base + u * TPW + group;
-      r.valid[u] = tok < t_end;
-      r.kq[u] = make_uint4(0, 0, 0, 0);
-      r.vq[u] = make_uint4(0, 0, 0, 0);
-      r.ks[u] = r.vs[u] = 1.f;
-      if (r.valid[u]) {
-        const int blk = table[tok / PAGE];
-        const size_t a = (static_cast<size_t>(blk) * PAGE + tok % PAGE) * tok_stride;
-        r.kq[u] = *reinterpret_cast<const uint4*>(kc + a);
-        r.vq[u] = *reinterpret_cast<const uint4*>(vc + a);
-        if (FP8) {
-          r.ks[u] = k_scale[static_cast<size_t>(blk) * Hkv + kvh];
-          r.vs[u] = v_scale[static_cast<size_t>(blk) * Hkv + kvh];
-        }
-      }
-    }
-  };
-  auto consume = [&](const Rows& r) {
-    const uint4* kq = r.kq;
-    const uint4* vq = r.vq;
-    const float* ks = r.ks;
-    const float* vs = r.vs;
-    const bool* valid = r.valid;
-    float sc[U][GH];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float kf[DPL];
-      dec_unpack<FP8>(kq[u], kf);
-#pragma unroll
-      for (int g = 0; g < GH; ++g) {
-        float d0 = 0.f;
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) d0 = fmaf(qr[g][d], kf[d], d0);
-#pragma unroll
-        for (int o = LPT / 2; o > 0; o >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-        sc[u][g] = valid[u] ? d0 * ks[u] : -INFINITY;
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < GH; ++g) {
-      float mn = m[g];
-#pragma unroll
-      for (int u = 0; u < U; ++u) mn = fmaxf(mn, sc[u][g]);
-      if (mn == -INFINITY) {   // this lane group has not seen a token yet: its weights are zero
-#pragma unroll
-        for (int u = 0; u < U; ++u) sc[u][g] = 0.f;
-        continue;
-      }
-      const float alpha = fast_exp2(m[g] - mn);
-      m[g] = mn;
-      float ps = 0.f;
-#pragma unroll
-      for (int d = 0; d < DPL; ++d) acc[g][d] *= alpha;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float p = fast_exp2(sc[u][g] - mn);
-        ps += p;
-        sc[u][g] = p * vs[u];
-      }
-      l[g] = l[g] * alpha + ps;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float vf[DPL];
-      dec_unpack<FP8>(vq[u], vf);
-#pragma unroll
-      for (int g = 0; g < GH; ++g)
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) acc[g][d] = fmaf(sc[u][g], vf[d], acc[g][d]);
-    }
-  };
+  int my_block = nz == 1 && warp + WARPS * lane < max_blocks ? table[warp + WARPS * lane] : 0;
+  uint32_t qa[16];   // the query head of rows r and r + 8 (both r % GP), in the order of the lane's key chunks
   {
-    constexpr int STEP = (DEC_THREADS / 32) * TPW * U;
-    int base = t_begin + warp * (TPW * U);
-    if (MODE >= 2) {
-      const uint32_t ring = smem_u32(dec_ring) + (warp * STAGES * U * 2 * 32 + lane) * 16;
-      auto issue = [&](int stage, int at) {
+    const int g = r % GP;
+    const __nv_bfloat16* qp = q + (static_cast<size_t>(b) * Hq + kvh * G + g) * HD;
+    const bool aligned = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int tok = at + u * TPW + group;
-          if (tok < t_end) {
-            const int blk = table[tok / PAGE];
-            const size_t a = (static_cast<size_t>(blk) * PAGE + tok % PAGE) * tok_stride;
-            const uint32_t dst = ring + ((stage * U + u) * 2) * 512;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(kc + a) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512), "l"(vc + a) : "memory");
-          }
+    for (int i = 0; i < 4; ++i) {
+      // bf16 rows: chunk c + 4 i is 8 dims; fp8 rows: chunk c + 4 (i / 2) is 16 dims, two vectors
+      const int v = FP8 ? (c + 4 * (i >> 1)) * 2 + (i & 1) : c + 4 * i;
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      if (g < G) {
+        if (aligned) {
+          w = *reinterpret_cast<const uint4*>(qp + 8 * v);
+        } else {
+          const unsigned short* h = reinterpret_cast<const unsigned short*>(qp + 8 * v);
+          w = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");   // one group per stage, empty ones included
-      };
-#pragma unroll
-      for (int s = 0; s < STAGES - 1; ++s) issue(s, base + s * STEP);
-      int slot = 0;
-      for (; base < t_end; base += STEP) {
-        issue(slot == 0 ? STAGES - 1 : slot - 1, base + (STAGES - 1) * STEP);
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
-        Rows r;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int tok = base + u * TPW + group;
-          r.valid[u] = tok < t_end;
-          r.kq[u] = make_uint4(0, 0, 0, 0);
-          r.vq[u] = make_uint4(0, 0, 0, 0);
-          r.ks[u] = r.vs[u] = 1.f;
-          if (r.valid[u]) {
-            const uint32_t src = ring + ((slot * U + u) * 2) * 512;
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(r.kq[u].x), "=r"(r.kq[u].y), "=r"(r.kq[u].z), "=r"(r.kq[u].w)
-                         : "r"(src));
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(r.vq[u].x), "=r"(r.vq[u].y), "=r"(r.vq[u].z), "=r"(r.vq[u].w)
-                         : "r"(src + 512));
-            if (FP8) {
-              const int blk = table[tok / PAGE];
-              r.ks[u] = k_scale[static_cast<size_t>(blk) * Hkv + kvh];
-              r.vs[u] = v_scale[static_cast<size_t>(blk) * Hkv + kvh];
-            }
-          }
-        }
-        consume(r);
-        slot = slot + 1 == STAGES ? 0 : slot + 1;
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    } else {
-      for (; base < t_end; base += STEP) {
-        Rows r;
-        load_rows(r, base);
-        consume(r);
-      }
+      qa[4 * i] = w.x;
+      qa[4 * i + 1] = w.y;
+      qa[4 * i + 2] = w.z;
+      qa[4 * i + 3] = w.w;
     }
   }
+  int ctx = context_lens[b], t_begin, t_end;
+  if (clustered) {
+    ctx = min(ctx, partition);
+    const int per = ((ctx + PAGE - 1) / PAGE + nz - 1) / nz * PAGE;
+    t_begin = min(z * per, ctx);
+    t_end = min(t_begin + per, ctx);
+  } else {
+    t_begin = z * partition;
+    t_end = min(ctx, t_begin + partition);
+  }
+  const int tiles = t_end > t_begin ? (t_end - t_begin + PAGE - 1) / PAGE : 0;
+  table += t_begin / PAGE;
+  const size_t tok_stride = static_cast<size_t>(Hkv) * Cfg::ROW;
+  const uint8_t* kc = static_cast<const uint8_t*>(k_cache) + static_cast<size_t>(kvh) * Cfg::ROW;
+  const uint8_t* vc = static_cast<const uint8_t*>(v_cache) + static_cast<size_t>(kvh) * Cfg::ROW;
+  const uint32_t ring = smem_u32(dec_ring) + warp * Cfg::RING;
 
-  // merge the lane groups of the warp, then the warps
+  // copies of this warp's i-th page (tile warp + 4 i); the table entries of 32 pages are read together
+  auto issue = [&](int i) {
+    const int tile = warp + WARPS * i;
+    if ((i & 31) == 0 && (i > 0 || nz > 1)) {
+      const int ahead = tile + WARPS * lane;
+      my_block = ahead < tiles ? table[ahead] : 0;
+    }
+    const int blk = __shfl_sync(0xffffffffu, my_block, i & 31);
+    if (tile < tiles) {
+      const uint32_t dst0 = ring + (i % Cfg::STAGES) * (2 * Cfg::TILE);
+      const size_t page = static_cast<size_t>(blk) * PAGE * tok_stride;
 #pragma unroll
-  for (int o = LPT; o < 32; o <<= 1) {
-#pragma unroll
-    for (int g = 0; g < GH; ++g) {
-      const float mo = __shfl_xor_sync(0xffffffffu, m[g], o);
-      const float lo = __shfl_xor_sync(0xffffffffu, l[g], o);
-      const float mn = fmaxf(m[g], mo);
-      const float wa = mn == -INFINITY ? 0.f : fast_exp2(m[g] - mn);
-      const float wb = mn == -INFINITY ? 0.f : fast_exp2(mo - mn);
-#pragma unroll
-      for (int d = 0; d < DPL; ++d) {
-        const float ao = __shfl_xor_sync(0xffffffffu, acc[g][d], o);
-        acc[g][d] = acc[g][d] * wa + ao * wb;
+      for (int u = 0; u < PAGE * Cfg::CPR / 32; ++u) {
+        const int row = (u * 32 + lane) / Cfg::CPR, ch = lane % Cfg::CPR;
+        const bool valid = t_begin + tile * PAGE + row < t_end;   // rows past the end become zeros
+        const size_t src = page + (valid ? row : 0) * tok_stride + ch * 16;
+        const uint32_t dst = dst0 + row * Cfg::ROW + ((ch ^ Cfg::swz(row)) << 4);
+        const int bytes = valid ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(kc + src), "r"(bytes) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + Cfg::TILE), "l"(vc + src), "r"(bytes) : "memory");
       }
-      l[g] = l[g] * wa + lo * wb;
-      m[g] = mn;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // one group per page, empty ones included
+  };
+#pragma unroll
+  for (int i = 0; i < Cfg::STAGES - 1; ++i) issue(i);
+
+  float qscale = scale * DEC_LOG2E;
+  {
+    if (FP8) {
+      float amax = 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 f = unpack_bf16x2(qa[i]);
+        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+      }
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+      const int e = min(max(static_cast<int>(__float_as_uint(amax) >> 23), 127 - 100), 127 + 100);   // biased exponent
+      const float to = __uint_as_float(static_cast<uint32_t>(127 + 13 + 127 - e) << 23);             // 2^(13 - (e - 127))
+      qscale *= __uint_as_float(static_cast<uint32_t>(e - 13) << 23);                               // its reciprocal
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 f = unpack_bf16x2(qa[i]);
+        qa[i] = dec_pack<true>(f.x * to, f.y * to);
+      }
     }
   }
-  if (group == 0) {
+  const int part_a = r / GP, part_b = part_a + 8 / GP;
+  float acc[16][4];
 #pragma unroll
-    for (int g = 0; g < GH; ++g) {
+  for (int j = 0; j < 16; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  float m = -INFINITY, l = 0.f, my_ks = 1.f, my_vs = 1.f;
+  int ev = 1;   // fp8: largest biased exponent of the value scales so far (acc is scaled by its inverse)
+
+  for (int i = 0; warp + WARPS * i < tiles; ++i) {
+    issue(i + Cfg::STAGES - 1);
+    float ks = 1.f, vs = 1.f;
+    if (FP8) {
+      if ((i & 31) == 0) {
+        const int ahead = warp + WARPS * (i + lane);
+        if (ahead < tiles) {
+          const size_t at = static_cast<size_t>(table[ahead]) * Hkv + kvh;
+          my_ks = k_scale[at];
+          my_vs = v_scale[at];
+        }
+      }
+      ks = __shfl_sync(0xffffffffu, my_ks, i & 31);
+      vs = __shfl_sync(0xffffffffu, my_vs, i & 31);
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(Cfg::STAGES - 1) : "memory");
+    __syncwarp();
+    const uint32_t kt = ring + (i % Cfg::STAGES) * (2 * Cfg::TILE), vt = kt + Cfg::TILE;
+    const int left = t_end - t_begin - (warp + WARPS * i) * PAGE;   // valid tokens of the page, from 1
+    // ---- scores of tokens 2c, 2c+1 (s[0], s[1]) and 2c+8, 2c+9 (s[2], s[3])
+    float s[4];
 #pragma unroll
-      for (int d = 0; d < DPL; ++d) sAcc[warp][g][sub * DPL + d] = acc[g][d];
-      if (sub == 0) {
-        sM[warp][g] = m[g];
-        sL[warp][g] = l[g];
+    for (int nt = 0; nt < 2; ++nt) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      const int t = nt * 8 + r;
+#pragma unroll
+      for (int u = 0; u < Cfg::CPR / 4; ++u) {
+        const uint4 w4 = dec_lds(kt + t * Cfg::ROW + (((c + 4 * u) ^ Cfg::swz(t)) << 4));
+        const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+        if (FP8) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int j = 4 * u + k;
+            dec_mma<FP8>(d, qa[2 * j], qa[2 * j], qa[2 * j + 1], qa[2 * j + 1], dec_fp8x2(w[k]), dec_fp8x2(w[k] >> 16));
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int j = 2 * u + k;
+            dec_mma<FP8>(d, qa[2 * j], qa[2 * j], qa[2 * j + 1], qa[2 * j + 1], w[2 * k], w[2 * k + 1]);
+          }
+        }
+      }
+      s[2 * nt] = d[0];
+      s[2 * nt + 1] = d[1];
+    }
+    const float f = qscale * ks;
+    float mx = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int t = 2 * c + (k & 1) + (k >> 1) * 8;
+      s[k] = t < left ? s[k] * f : -INFINITY;
+      mx = fmaxf(mx, s[k]);
+    }
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float mn = fmaxf(m, mx);
+    float back = 1.f;
+    if (FP8) {
+      const int e = min(max(static_cast<int>((__float_as_uint(vs) >> 23) & 255u), ev), 253);
+      back = e - ev > 126 ? 0.f : __uint_as_float(static_cast<uint32_t>(127 - (e - ev)) << 23);
+      ev = e;
+      vs *= 16384.f * __uint_as_float(static_cast<uint32_t>(254 - e) << 23);
+    }
+    if (__any_sync(0xffffffffu, mn != m || back != 1.f)) {
+      const float alpha = mn == -INFINITY ? 0.f : fast_exp2(m - mn);
+      l *= alpha;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[j][k] *= alpha * back;
+      m = mn;
+    }
+    const float base = mn == -INFINITY ? 0.f : mn;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      s[k] = fast_exp2(s[k] - base);
+      l += s[k];
+      s[k] *= vs;
+    }
+    const uint32_t a0 = dec_part<FP8>(s[0], s[1], part_a), a2 = dec_part<FP8>(s[2], s[3], part_a);
+    const uint32_t a1 = GP >= 4 ? dec_part<FP8>(s[0], s[1], part_b) : 0u, a3 = GP >= 4 ? dec_part<FP8>(s[2], s[3], part_b) : 0u;
+    const uint32_t x0 = GP == 8 ? dec_part<FP8>(s[0], s[1], 2) : 0u, x2 = GP == 8 ? dec_part<FP8>(s[2], s[3], 2) : 0u;
+    // ---- output dims 16 n + j of n-tile j
+#pragma unroll
+    for (int h = 0; h < Cfg::CPR / 8; ++h) {
+      uint32_t w[4][4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int t = 2 * c + (k & 1) + (k >> 1) * 8;
+        const uint4 w4 = dec_lds(vt + t * Cfg::ROW + (((r * (Cfg::CPR / 8) + h) ^ Cfg::swz(t)) << 4));
+        w[k][0] = w4.x;
+        w[k][1] = w4.y;
+        w[k][2] = w4.z;
+        w[k][3] = w4.w;
+      }
+#pragma unroll
+      for (int jj = 0; jj < (FP8 ? 16 : 8); ++jj) {
+        uint32_t b0, b1;
+        if (FP8) {   // byte jj of tokens 2c and 2c+1, of 2c+8 and 2c+9
+          const uint32_t pick = (jj & 3) | ((4 + (jj & 3)) << 4);
+          b0 = dec_fp8x2(__byte_perm(w[0][jj >> 2], w[1][jj >> 2], pick));
+          b1 = dec_fp8x2(__byte_perm(w[2][jj >> 2], w[3][jj >> 2], pick));
+        } else {     // half jj
+          const uint32_t pick = (jj & 1) ? 0x7632u : 0x5410u;
+          b0 = __byte_perm(w[0][jj >> 1], w[1][jj >> 1], pick);
+          b1 = __byte_perm(w[2][jj >> 1], w[3][jj >> 1], pick);
+        }
+        const int j = h * 8 + jj;
+        dec_mma<FP8>(acc[j], a0, a1, a2, a3, b0, b1);
+        if (GP == 8) dec_mma<FP8>(acc[j], x0, 0u, x2, 0u, b0, b1);
       }
     }
+    __syncwarp();   // every lane has read the stage before its next copies are issued
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+
+  // ---- the parts of a head: rows r and r + 8, then rows GP apart; then the warps through shared memory
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  const float unit = FP8 ? __uint_as_float(static_cast<uint32_t>(ev) << 23) * (1.f / 16384.f) : 1.f;
+  // per warp [GP][PITCH], channel 16 n + j at 8 j + n (what the lanes of a row hold is then adjacent), then maxima and sums
+  constexpr int PITCH = HD + 8;
+  float* wo = reinterpret_cast<float*>(dec_ring + warp * Cfg::RING);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    float o0 = acc[j][0] + acc[j][2], o1 = acc[j][1] + acc[j][3];
+#pragma unroll
+    for (int d = 16; d >= 4 * GP; d >>= 1) {
+      o0 += __shfl_xor_sync(0xffffffffu, o0, d);
+      o1 += __shfl_xor_sync(0xffffffffu, o1, d);
+    }
+    if (r < GP) {
+      *reinterpret_cast<float2*>(wo + r * PITCH + 8 * j + 2 * c) = make_float2(o0 * unit, o1 * unit);
+    }
+  }
+  if (r < GP && c == 0) {
+    wo[GP * PITCH + r] = m;
+    wo[GP * PITCH + GP + r] = l;
   }
   __syncthreads();
-#pragma unroll
-  for (int g = 0; g < GH; ++g) {
+  for (int e = tid; e < G * HD; e += (WARPS * 32)) {
+    const int g = e / HD, at = e % HD, d = (at & 7) * 16 + (at >> 3);
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < DEC_THREADS / 32; ++w) M = fmaxf(M, sM[w][g]);
+    for (int w = 0; w < WARPS; ++w) M = fmaxf(M, reinterpret_cast<const float*>(dec_ring + w * Cfg::RING)[GP * PITCH + g]);
     float L = 0.f, o = 0.f;
 #pragma unroll
-    for (int w = 0; w < DEC_THREADS / 32; ++w) {
-      const float wgt = sM[w][g] == -INFINITY ? 0.f : fast_exp2(sM[w][g] - M);
-      L += sL[w][g] * wgt;
-      o += sAcc[w][g][tid] * wgt;
+    for (int w = 0; w < WARPS; ++w) {
+      const float* p = reinterpret_cast<const float*>(dec_ring + w * Cfg::RING);
+      const float mw = p[GP * PITCH + g];
+      const float wgt = mw == -INFINITY ? 0.f : fast_exp2(mw - M);
+      L += p[GP * PITCH + GP + g] * wgt;
+      o += p[g * PITCH + at] * wgt;
     }
-    const int head = head0 + g;
-    if (nsplit == 1) {
-      out[(static_cast<size_t>(b) * Hq + head) * HD + tid] = __float2bfloat16(L > 0.f ? o / L : 0.f);
+    const int head = kvh * G + g;
+    if (nz == 1) {
+      out[(static_cast<size_t>(b) * Hq + head) * HD + d] = __float2bfloat16(L > 0.f ? o / L : 0.f);
+    } else if (clustered) {
+      sO[g][d] = o;
+      if (d == 0) {
+        sM[g] = M;
+        sL[g] = L;
+      }
     } else {
-      part_o[((static_cast<size_t>(b) * Hq + head) * nsplit + split) * HD + tid] = o;
-      if (tid == 0) {
-        float* ml = part_ml + ((static_cast<size_t>(b) * Hq + head) * nsplit + split) * 2;
+      part_o[((static_cast<size_t>(b) * Hq + head) * nz + z) * HD + d] = o;
+      if (d == 0) {
+        float* ml = part_ml + ((static_cast<size_t>(b) * Hq + head) * nz + z) * 2;
         ml[0] = M * DEC_LN2;   // natural-log domain for the merge kernel
         ml[1] = L;
       }
     }
   }
+  if (!clustered || nz == 1) return;
+  // ---- the heads' channels are dealt to the CTAs, which add up the cluster's parts
+  dec_cluster_sync();
+  for (int e = z * (WARPS * 32) + tid; e < G * HD; e += nz * (WARPS * 32)) {
+    const int g = e / HD, d = e % HD;
+    float M = -INFINITY, mz[DEC_MAX_CLUSTER], lz[DEC_MAX_CLUSTER], oz[DEC_MAX_CLUSTER], L = 0.f, o = 0.f;
+#pragma unroll
+    for (int k = 0; k < DEC_MAX_CLUSTER; ++k) {
+      mz[k] = k < nz ? dec_ld_cluster(smem_u32(&sM[g]), k) : -INFINITY;
+      lz[k] = k < nz ? dec_ld_cluster(smem_u32(&sL[g]), k) : 0.f;
+      oz[k] = k < nz ? dec_ld_cluster(smem_u32(&sO[g][d]), k) : 0.f;
+      M = fmaxf(M, mz[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < DEC_MAX_CLUSTER; ++k) {
+      const float wgt = mz[k] == -INFINITY ? 0.f : fast_exp2(mz[k] - M);
+      L += lz[k] * wgt;
+      o += oz[k] * wgt;
+    }
+    out[(static_cast<size_t>(b) * Hq + kvh * G + g) * HD + d] = __float2bfloat16(L > 0.f ? o / L : 0.f);
+  }
+  dec_cluster_sync();   // nobody leaves while its shared memory is read
 }
 
 // Exact merge of split-KV partials: out = sum_i acc_i e^{m_i - M} / sum_i l_i e^{m_i - M}.
@@ -498,51 +609,61 @@ B2_EXPORT int b2_paged_decode(const void* q, const void* k_cache, const void* v_
   }
   if (B <= 0) return 0;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const int G = Hq / Hkv;
-  // query heads per CTA (their q pieces and accumulators live in registers: fp8 rows put 16 dims on a
-  // lane, so four heads would leave room for only two CTAs per SM)
-  const int GH = (G % 4 == 0 && !fp8) ? 4 : (G % 2 == 0 ? 2 : 1);
-  dim3 grid(B, Hkv * (G / GH), nsplit);
-  // B200FW_DECODE_MODE selects the row loop: 0 registers, 3 the cp.async ring (read on every call, so that one
-  // process can compare them)
-  const int mode = [] {
-    const char* e = std::getenv("B200FW_DECODE_MODE");
-    if (e != nullptr && (e[0] == '0' || e[0] == '3')) return e[0] - '0';
-    return DEC_DEFAULT_MODE;
-  }();
-#define B2_DECODE_LAUNCH_M(F8, GHV, MD)                                                                    \
-  do {                                                                                                     \
-    constexpr int ring = MD >= 2 ? (DEC_THREADS / 32) * MD * DEC_UNROLL * 2 * 512 : 0;                     \
-    auto kern = paged_decode_kernel<F8, GHV, MD>;                                                          \
-    if (ring > 0) {                                                                                        \
-      static bool attr_set[64] = {};                                                                       \
-      int dev = 0;                                                                                         \
-      cudaGetDevice(&dev);                                                                                 \
-      if (!attr_set[dev & 63]) {                                                                           \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring);                     \
-        attr_set[dev & 63] = true;                                                                         \
-      }                                                                                                    \
-    }                                                                                                      \
-    kern<<<grid, DEC_THREADS, ring, stream>>>(                                                             \
-        static_cast<const __nv_bfloat16*>(q), k_cache, v_cache, k_scale, v_scale, block_tables, context_lens, \
-        max_blocks, static_cast<__nv_bfloat16*>(out), part_o, part_ml, Hq, Hkv, partition, scale);         \
+  const int G = Hq / Hkv, GP = G > 4 ? 8 : G > 2 ? 4 : G;
+  // Without a split from the caller, the CTAs of a cluster share a context: as many (up to 8) as keep the grid within two CTAs
+  // per SM, i.e. in one wave, and no more than the table has pieces of 64 tokens.  Clusters of 1 / 2 / 4 / 8, us: 8 (sequence, kv
+  // head) pairs of 1024 tokens 12.9 / 9.6 / 7.6 / 6.3; 64 pairs of up to 8192 80.3 / 45.5 / 41.8 / 45.5; 256 pairs of up to 2000
+  // 41.3 / 48.2 / 58.5 / 87.4.
+  int cluster = 1;
+  if (nsplit == 1)
+    while (cluster < DEC_MAX_CLUSTER && static_cast<long long>(B) * Hkv * cluster * 2 <= 2LL * num_sms() && cluster * 2 * (DEC_CHUNK / PAGE) <= max_blocks)
+      cluster *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(B, Hkv, nsplit == 1 ? cluster : nsplit);
+  // Two warps per CTA where there are many pairs anyway: CTAs of short contexts come and go faster.  256 sequences, 8 kv
+  // heads, two / four warps, us: 128 tokens 31 / 39, 1024 tokens 130 / 125; 32 sequences of 2000 tokens 53 / 41.
+  const int warps = static_cast<long long>(B) * Hkv >= 8LL * num_sms() ? 2 : 4;
+  cfg.blockDim = dim3(warps * 32, 1, 1);
+  cfg.dynamicSmemBytes = warps * (fp8 ? DecCfg<true>::RING : DecCfg<false>::RING);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = cluster;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+#define B2_DECODE_LAUNCH_W(F8, GPV, WV)                                                                                   \
+  do {                                                                                                              \
+    auto kern = paged_decode_kernel<F8, GPV, WV>;                                                                   \
+    static bool attr_set[64] = {};                                                                                  \
+    int dev = 0;                                                                                                    \
+    cudaGetDevice(&dev);                                                                                            \
+    if (!attr_set[dev & 63]) {                                                                                      \
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WV * DecCfg<F8>::RING);                \
+      attr_set[dev & 63] = true;                                                                                    \
+    }                                                                                                               \
+    cudaLaunchKernelEx(&cfg, kern, static_cast<const __nv_bfloat16*>(q), k_cache, v_cache, k_scale, v_scale,        \
+                       block_tables, context_lens, max_blocks, static_cast<__nv_bfloat16*>(out), part_o, part_ml,   \
+                       Hq, Hkv, partition, scale, nsplit == 1 ? 1 : 0);                                             \
   } while (0)
-#define B2_DECODE_LAUNCH(F8, GHV)                                                                          \
-  do {                                                                                                     \
-    if (mode == 3) B2_DECODE_LAUNCH_M(F8, GHV, 3);                                                         \
-    else B2_DECODE_LAUNCH_M(F8, GHV, 0);                                                                   \
+#define B2_DECODE_LAUNCH(F8, GPV)                     \
+  do {                                                \
+    if (warps == 2) B2_DECODE_LAUNCH_W(F8, GPV, 2);   \
+    else B2_DECODE_LAUNCH_W(F8, GPV, 4);              \
   } while (0)
-  if (fp8) {
-    if (GH == 4) B2_DECODE_LAUNCH(true, 4);
-    else if (GH == 2) B2_DECODE_LAUNCH(true, 2);
-    else B2_DECODE_LAUNCH(true, 1);
-  } else {
-    if (GH == 4) B2_DECODE_LAUNCH(false, 4);
-    else if (GH == 2) B2_DECODE_LAUNCH(false, 2);
-    else B2_DECODE_LAUNCH(false, 1);
-  }
-#undef B2_DECODE_LAUNCH_M
+#define B2_DECODE_GROUP(F8)                       \
+  do {                                            \
+    if (GP == 8) B2_DECODE_LAUNCH(F8, 8);         \
+    else if (GP == 4) B2_DECODE_LAUNCH(F8, 4);    \
+    else if (GP == 2) B2_DECODE_LAUNCH(F8, 2);    \
+    else B2_DECODE_LAUNCH(F8, 1);                 \
+  } while (0)
+  if (fp8) B2_DECODE_GROUP(true);
+  else B2_DECODE_GROUP(false);
+#undef B2_DECODE_GROUP
 #undef B2_DECODE_LAUNCH
+#undef B2_DECODE_LAUNCH_W
   B2_LAUNCH_CHECK("paged_decode");
   if (nsplit > 1) {
     paged_merge_kernel<<<B * Hq, HD, 0, stream>>>(part_o, part_ml, static_cast<__nv_bfloat16*>(out), lse, nsplit);

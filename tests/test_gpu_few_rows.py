@@ -1,0 +1,81 @@
+"""Decode attention and products with few rows against 64-bit references, at the sizes where their splits change."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _error(got, want):
+    """Relative error in the 2-norm, and that of the 64-bit result rounded to bf16 (which no bf16 output can do without)."""
+    want = want.double().cpu()
+    d = lambda t: float((t.double().cpu() - want).norm() / want.norm().clamp(min=1e-30))
+    return d(got), d(want.to(torch.bfloat16))
+
+
+def _decode_reference(q, kc, vc, bt, lens, Hq, ks, vs):
+    Hkv = kc.shape[2]
+    K, V = (t.view(torch.float8_e4m3fn).double() * s.double()[:, None, :, None] if s is not None else t.double()
+            for t, s in ((kc, ks), (vc, vs)))
+    out = torch.zeros(q.shape, dtype=torch.float64, device=DEV)
+    for b, n in enumerate(lens):
+        if n:
+            pos = torch.arange(n, device=DEV)
+            at = bt[b, pos // 16].long() * 16 + pos % 16
+            k, v = K.reshape(-1, Hkv, 128)[at], V.reshape(-1, Hkv, 128)[at]
+            s = torch.einsum("hgd,nhd->hgn", q[b].double().reshape(Hkv, Hq // Hkv, 128), k) / math.sqrt(128)
+            out[b] = torch.einsum("hgn,nhd->hgd", s.softmax(-1), v).reshape(-1)
+    return out
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("Hq,Hkv", [(2, 2), (4, 2), (6, 2), (8, 2), (5, 1), (8, 1)])     # 1, 2, 3, 4, 5 and 8 heads per kv head
+@pytest.mark.parametrize("lens", [[1], [0, 5, 16, 17], [63, 64, 65, 130, 257], [2000, 1]])
+def test_decode_attention_over_clusters(fp8, Hq, Hkv, lens):
+    """Contexts of no token, of less than a page and of unequal parts; pages past the end hold NaN; scales differ per page."""
+    from b200fw.ops import paged_decode_attention
+    g = torch.Generator(device=DEV).manual_seed(1)
+    need = [-(-n // 16) for n in lens]
+    blocks = sum(need) + 1
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    kc, vc = rnd(blocks, 16, Hkv, 128), rnd(blocks, 16, Hkv, 128)
+    perm = torch.randperm(blocks - 1, device=DEV, generator=g)
+    bt = torch.full((len(lens), 160), -1, dtype=torch.int32, device=DEV)
+    at = 0
+    for b, n in enumerate(need):
+        bt[b, :n] = perm[at:at + n].int()
+        if lens[b] % 16:      # rows past the end of the context
+            kc[bt[b, n - 1].long(), lens[b] % 16:] = math.nan
+            vc[bt[b, n - 1].long(), lens[b] % 16:] = math.nan
+        at += n
+    ks = vs = None
+    if fp8:
+        kc, vc = (t.to(torch.float8_e4m3fn).view(torch.uint8) for t in (kc, vc))
+        ks, vs = (10.0 ** (-4 + 4 * torch.rand(blocks, Hkv, device=DEV, generator=g)) for _ in range(2))
+    else:
+        kc, vc = kc.to(torch.bfloat16), vc.to(torch.bfloat16)
+    q = rnd(len(lens), Hq * 128).to(torch.bfloat16)
+    cl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    want = _decode_reference(q, kc, vc, bt, lens, Hq, ks, vs)
+    for part, nsplit in ((0, 1), (64, max(1, -(-max(lens) // 64)))):
+        got, floor = _error(paged_decode_attention(q, kc, vc, bt, cl, Hq, k_scale=ks, v_scale=vs, partition=part, nsplit=nsplit), want)
+        # rounding the output, plus 32-bit scores of up to about 30 and their exponentials
+        assert got <= 1.02 * floor + 2e-5, (part, nsplit, got, floor)
+
+
+def test_decode_attention_of_many_pairs_and_unaligned_queries():
+    """So many (sequence, kv head) pairs that CTAs of two warps run; queries two bytes off a vector's alignment."""
+    from b200fw.ops import paged_decode_attention
+    g = torch.Generator(device=DEV).manual_seed(2)
+    B, Hq, Hkv = 300, 8, 4
+    lens = torch.randint(1, 70, (B,), generator=torch.Generator().manual_seed(3)).tolist()
+    kc, vc = (torch.randn(B * 5, 16, Hkv, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    bt = torch.arange(B * 5, device=DEV, dtype=torch.int32).reshape(B, 5)
+    flat = torch.randn(B * Hq * 128 + 1, device=DEV, generator=g).to(torch.bfloat16)
+    q = flat[1:].view(B, Hq * 128)
+    cl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    got, floor = _error(paged_decode_attention(q, kc, vc, bt, cl, Hq), _decode_reference(q, kc, vc, bt, lens, Hq, None, None))
+    assert got <= 1.02 * floor + 2e-5, (got, floor)
