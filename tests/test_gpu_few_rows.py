@@ -79,3 +79,49 @@ def test_decode_attention_of_many_pairs_and_unaligned_queries():
     cl = torch.tensor(lens, dtype=torch.int32, device=DEV)
     got, floor = _error(paged_decode_attention(q, kc, vc, bt, cl, Hq), _decode_reference(q, kc, vc, bt, lens, Hq, None, None))
     assert got <= 1.02 * floor + 2e-5, (got, floor)
+
+
+@pytest.mark.parametrize("b_mn", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 1024), (7, 776, 1032), (128, 200, 2056), (300, 72, 1544)])
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("cluster", [1, 2, 4, 8])
+def test_cluster_products(b_mn, M, N, K, bn, cluster):
+    """Every tile width and cluster size, whatever the shape would choose: bf16 and fp32 outputs, residual, accumulation."""
+    from b200fw import _native as nv
+    g = torch.Generator(device=DEV).manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    a, b, r = rnd(M, K).to(torch.bfloat16), rnd(*((K, N) if b_mn else (N, K))).to(torch.bfloat16), rnd(M, N).to(torch.bfloat16)
+    prod = a.double() @ (b.double() if b_mn else b.double().t())
+    wide = torch.zeros(M, N + 8, device=DEV, dtype=torch.bfloat16)     # a strided output: nothing past its columns
+    f32 = rnd(M, N)
+    acc = r.clone()
+    for out, res, flags, want in ((wide[:, :N], None, 0, prod), (torch.empty_like(r), r, 4, prod + r.double()),
+                                  (acc, None, 2, prod + r.double()), (f32, None, 3, prod + f32.double())):
+        nv.check(nv.lib().b2_gemm_bf16_cluster(nv.ptr(a), nv.ptr(b), nv.ptr(out), nv.ptr(res), M, N, K, a.stride(0), b.stride(0),
+                                               out.stride(0), b_mn, flags, bn, cluster, 0, 0, nv.stream_ptr()), "cluster")
+        got, floor = _error(out, want)
+        # 32-bit sums of K terms in a fixed order: well below sqrt(K) * 2^-24 of the result, 1e-5 with room to spare
+        assert got <= (1.02 * floor if flags != 3 else 0.0) + 1e-5, (flags, got, floor)
+    assert float(wide[:, N:].abs().max()) == 0.0
+    nv.assert_ok()
+
+
+@pytest.mark.parametrize("act", ["silu", "relu2"])
+@pytest.mark.parametrize("M", [1, 33, 256])
+def test_products_with_few_rows_take_every_epilogue(act, M):
+    """Through the public entry points, at a shape that the dispatch gives to clusters, against the persistent kernel too."""
+    from b200fw.ops import gemm
+    from b200fw.ops.gemm import linear_act
+    g = torch.Generator(device=DEV).manual_seed(5)
+    a, b = (torch.randn(*s, device=DEV, generator=g).mul(0.2).to(torch.bfloat16) for s in ((M, 3072), (1024, 3072)))
+    prod = a.double() @ b.double().t()
+    z = prod[:, :520]
+    want = prod.clone()
+    want[:, :520] = z * torch.sigmoid(z) if act == "silu" else z.clamp(min=0) ** 2
+    got, floor = _error(linear_act(a, b, act, 520), want)
+    assert got <= 1.05 * floor + 2e-5, (got, floor)
+    got, floor = _error(gemm(a, b), prod)
+    assert got <= 1.02 * floor + 1e-5
+    got, floor = _error(gemm(a, b, bn=128), prod)       # a given width keeps the persistent kernel
+    assert got <= 1.02 * floor + 1e-5
+    assert torch.equal(gemm(a, b), gemm(a, b))
