@@ -45,6 +45,11 @@ class _RMSNorm(torch.autograd.Function):
         dy = dy.contiguous()
         dx = torch.empty_like(x)
         L = nv.lib()
+        if not ctx.needs_input_grad[1] and getattr(w, "main_grad", None) is None and H <= 4096:      # frozen: no column sums
+            nv.check(L.b2_rmsnorm_bwd(nv.ptr(dy), nv.ptr(x), nv.ptr(w), nv.ptr(rstd), nv.ptr(dx), nv.ptr(None), nv.ptr(None),
+                                      M, H, 0, 0, 0, nv.stream_ptr()), "rmsnorm_bwd")
+            nv.count_launch()
+            return dx, None, None
         partial = torch.empty(L.b2_rmsnorm_bwd_ctas() * H, device=x.device, dtype=torch.float32)
 
         def run(out, acc):
@@ -52,7 +57,7 @@ class _RMSNorm(torch.autograd.Function):
             nv.check(L.b2_rmsnorm_bwd(nv.ptr(dy), nv.ptr(x), nv.ptr(w), nv.ptr(rstd), nv.ptr(dx),
                                       nv.ptr(tgt), nv.ptr(partial), M, H, 0, int(acc),
                                       int(tgt.dtype == torch.float32), nv.stream_ptr()), "rmsnorm_bwd")
-            nv.count_launch(3)
+            nv.count_launch(2)
             return tgt
 
         dw = grad_into_main(w, run)

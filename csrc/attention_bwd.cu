@@ -23,21 +23,44 @@ constexpr int ATB_THREADS = 352;  // warp 0 TMA, warps 1 and 10 MMA issue, warps
 constexpr float LOG2E = 1.4426950408889634f;
 
 // ---------------------------------------------------------------------------------------------
-__global__ void attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
-                                     const __nv_bfloat16* __restrict__ d_o, float* __restrict__ D,
-                                     long long T, int Hq) {
-  const long long gw = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= T * Hq) return;
-  const long long t = gw / Hq;
-  const int h = static_cast<int>(gw % Hq);
-  const size_t off = (static_cast<size_t>(t) * Hq + h) * 128 + lane * 4;
-  uint2 a = *reinterpret_cast<const uint2*>(o + off);
-  uint2 b = *reinterpret_cast<const uint2*>(d_o + off);
-  float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y);
-  float s = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
-  s = warp_sum(s);
-  if (lane == 0) D[static_cast<size_t>(h) * T + t] = s;
+// A row (one token, one head) is 16 lanes of 16 bytes; a warp takes 8 rows that lie one after the other and requests all of them
+// before it uses the first.  (A warp per row with 8-byte accesses: 21 us for 8192 x 16 rows, twice its traffic; now 16.)
+constexpr int PREP_ROWS = 8;
+
+__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
+                                                            const __nv_bfloat16* __restrict__ d_o, float* __restrict__ D,
+                                                            long long T, int Hq) {
+  const int lane = threadIdx.x & 31, l16 = lane & 15, sub = lane >> 4;
+  const long long first = ((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * PREP_ROWS, rows = T * Hq;
+  if (first >= rows) return;
+  const bool wide = (reinterpret_cast<uintptr_t>(o) & 15) == 0;   // d_o is read by TMA too, o only here
+  uint4 a[PREP_ROWS / 2], b[PREP_ROWS / 2];
+#pragma unroll
+  for (int u = 0; u < PREP_ROWS / 2; ++u) {
+    const long long row = first + 2 * u + sub < rows ? first + 2 * u + sub : rows - 1;
+    const __nv_bfloat16* op = o + row * 128 + l16 * 8;
+    if (wide) {
+      a[u] = *reinterpret_cast<const uint4*>(op);
+    } else {
+      const uint2 lo = reinterpret_cast<const uint2*>(op)[0], hi = reinterpret_cast<const uint2*>(op)[1];
+      a[u] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+    }
+    b[u] = *reinterpret_cast<const uint4*>(d_o + row * 128 + l16 * 8);
+  }
+#pragma unroll
+  for (int u = 0; u < PREP_ROWS / 2; ++u) {
+    const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, bw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 x = unpack_bf16x2(aw[j]), y = unpack_bf16x2(bw[j]);
+      s = fmaf(x.x, y.x, fmaf(x.y, y.y, s));
+    }
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    const long long row = first + 2 * u + sub;
+    if (l16 == 0 && row < rows) D[static_cast<size_t>(row % Hq) * T + row / Hq] = s;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -787,7 +810,7 @@ B2_EXPORT int b2_attn_bwd(const void* q, const void* k, const void* v, const voi
   int* status = status_ptr();
   if (!status) return 3;
   {
-    const long long warps = static_cast<long long>(T) * Hq;
+    const long long warps = (static_cast<long long>(T) * Hq + PREP_ROWS - 1) / PREP_ROWS;
     attn_bwd_prep_kernel<<<static_cast<int>((warps + 7) / 8), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out), Dsum,
         static_cast<long long>(T), Hq);

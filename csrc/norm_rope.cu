@@ -28,6 +28,16 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<bf16x8*>(p) = r;
 }
 
+__device__ __forceinline__ void raw8(const uint4& q, float (&f)[8]) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = unpack_bf16x2(w[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
 template <int THREADS>
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
   v = warp_sum(v);
@@ -209,105 +219,98 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------
-// RMSNorm backward split in two high-occupancy kernels (H <= 2048):
-//   dx kernel: one warp per row, nothing carried across rows (few registers, many warps in flight);
-//   dw kernel: column reduction dw[h] = sum_r dy[r,h] * x[r,h] * rstd[r]; a thread owns 8 columns and
-//              strides over rows with four independent loads in flight; per-CTA partials.
-// x and dy are read twice, the second time from L2.
+// RMSNorm backward, one warp per row, rows up to 256 * NV columns held as they came (16-bit) until they are used.
+//   dx = rstd * (dy*w - xhat * mean(dy*w*xhat)),  dw = sum_rows dy * xhat,  xhat = x*rstd
+// Bound by HBM: x and dy are read once.  (Two kernels, one for dx and one for the column sums, read them twice: 33.5 us for
+// 8192 x 1024, now 16; a CTA per row, two block-wide sums per row on the critical path and two rows in flight per SM, took 57 us
+// for 4096 x 2560, now 22 with a frozen weight.)  The weight gradient stays in registers: each lane owns the same columns of every row it sees; the
+// warps of a CTA meet once, in shared memory, in order.  DW = false: a frozen weight, no column sums at all.
 // ---------------------------------------------------------------------------------------------
-template <int NV>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_dx_kernel(
+template <int NV, bool DW>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_rows_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
     const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
-    __nv_bfloat16* __restrict__ dx, int M, int H, int add_to_dx) {
-  const int lane = threadIdx.x & 31;
-  const int warps_per_grid = (gridDim.x * blockDim.x) >> 5;
+    __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, int M, int H, int add_to_dx) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = H / 8;
-  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < M; row += warps_per_grid) {
-    const __nv_bfloat16* xr = x + static_cast<size_t>(row) * H;
-    const __nv_bfloat16* dyr = dy + static_cast<size_t>(row) * H;
-    __nv_bfloat16* dxr = dx + static_cast<size_t>(row) * H;
+  float acc[DW ? NV : 1][8];
+  if (DW) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  }
+  for (int row = blockIdx.x * 8 + warp; row < M; row += gridDim.x * 8) {
+    const size_t off = static_cast<size_t>(row) * H;
+    uint4 xr[NV], gr[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = lane + i * 32;
+      xr[i] = gr[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (c < nvec) {
+        xr[i] = *reinterpret_cast<const uint4*>(x + off + c * 8);
+        gr[i] = *reinterpret_cast<const uint4*>(dy + off + c * 8);
+      }
+    }
     const float rstd = rstd_in[row];
-    float xh[NV][8], g[NV][8];
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int c = lane + i * 32;
       if (c < nvec) {
-        float dv[8], wv[8];
-        load8(xr + c * 8, xh[i]);
-        load8(dyr + c * 8, dv);
+        float xv[8], dv[8], wv[8];
+        raw8(xr[i], xv);
+        raw8(gr[i], dv);
         load8(w + c * 8, wv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] *= rstd;
-          g[i][j] = dv[j] * wv[j];
-          dot += g[i][j] * xh[i][j];
+          const float t = dv[j] * (xv[j] * rstd);
+          if (DW) acc[DW ? i : 0][j] += t;
+          dot = fmaf(t, wv[j], dot);
         }
       }
     }
     dot = warp_sum(dot) / H;
+    // the second pass unpacks again: 32-bit copies of the row kept from the first one would double the registers
+    const __nv_bfloat16* w2 = w;
+    asm volatile("" : "+l"(w2));
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
+      asm volatile("" : "+r"(xr[i].x), "+r"(xr[i].y), "+r"(xr[i].z), "+r"(xr[i].w), "+r"(gr[i].x), "+r"(gr[i].y), "+r"(gr[i].z), "+r"(gr[i].w));
       const int c = lane + i * 32;
       if (c < nvec) {
-        float o[8];
-        if (add_to_dx) load8(dxr + c * 8, o);
+        float xv[8], dv[8], wv[8], o[8];
+        raw8(xr[i], xv);
+        raw8(gr[i], dv);
+        load8(w2 + c * 8, wv);
+        if (add_to_dx) load8(dx + off + c * 8, o);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float d = rstd * (g[i][j] - xh[i][j] * dot);
+          const float d = rstd * (dv[j] * wv[j] - xv[j] * rstd * dot);
           o[j] = add_to_dx ? o[j] + d : d;
         }
-        store8(dxr + c * 8, o);
+        store8(dx + off + c * 8, o);
       }
     }
   }
-}
-
-__global__ void __launch_bounds__(256) rmsnorm_bwd_dw_kernel(
-    const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-    const float* __restrict__ rstd_in, float* __restrict__ dw_partial, int M, int H) {
-  // thread -> column vector c = threadIdx.x % nvec (nvec <= 256), row lane rl = threadIdx.x / nvec
-  const int nvec = H / 8;
-  const int rows_per_cta_step = blockDim.x / nvec;       // 1 for H=2048, 2 for H=1024, ...
-  const int c = threadIdx.x % nvec, rl = threadIdx.x / nvec;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const int stride = gridDim.x * rows_per_cta_step;
-  int row = blockIdx.x * rows_per_cta_step + rl;
-  if (rl < rows_per_cta_step) {
-    for (; row + 3 * stride < M; row += 4 * stride) {
-      float xv[4][8], dv[4][8], rs[4];
+  if (!DW) return;
+  extern __shared__ float sdw[];   // [8 warps][H]
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const size_t o = static_cast<size_t>(row + u * stride) * H + c * 8;
-        load8(x + o, xv[u]);
-        load8(dy + o, dv[u]);
-        rs[u] = rstd_in[row + u * stride];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] += dv[u][j] * xv[u][j] * rs[u];
-    }
-    for (; row < M; row += stride) {
-      float xv[8], dv[8];
-      const size_t o = static_cast<size_t>(row) * H + c * 8;
-      load8(x + o, xv);
-      load8(dy + o, dv);
-      const float rs = rstd_in[row];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += dv[j] * xv[j] * rs;
+  for (int i = 0; i < NV; ++i) {
+    const int c = lane + i * 32;
+    if (c < nvec) {
+      float4* p = reinterpret_cast<float4*>(sdw + static_cast<size_t>(warp) * H + c * 8);
+      p[0] = make_float4(acc[DW ? i : 0][0], acc[DW ? i : 0][1], acc[DW ? i : 0][2], acc[DW ? i : 0][3]);
+      p[1] = make_float4(acc[DW ? i : 0][4], acc[DW ? i : 0][5], acc[DW ? i : 0][6], acc[DW ? i : 0][7]);
     }
   }
-  extern __shared__ float sdw[];   // [H]
-  for (int i = threadIdx.x; i < H; i += blockDim.x) sdw[i] = 0.f;
   __syncthreads();
-  if (rl < rows_per_cta_step) {
+  for (int i = threadIdx.x; i < H; i += 256) {
+    float t = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(&sdw[c * 8 + j], acc[j]);
+    for (int k = 0; k < 8; ++k) t += sdw[static_cast<size_t>(k) * H + i];
+    dw_partial[static_cast<size_t>(blockIdx.x) * H + i] = t;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < H; i += blockDim.x) dw_partial[static_cast<size_t>(blockIdx.x) * H + i] = sdw[i];
 }
 
 // dw[h] (+)= sum_p partial[p, h]   (bf16 or fp32 destination)
@@ -355,6 +358,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
 // before the first is processed.  (A warp per (token, head) with 8-byte accesses and a dependent
 // position -> table load per unit ran at a third of the memory bandwidth.)
 constexpr int QKR_PAIRS = 4;
+constexpr int QKB_CTAS = 2;    // CTAs per SM of the backward kernel
 
 __device__ __forceinline__ void qkr_unpack8(const uint4& q, float* f) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
@@ -457,7 +461,9 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(
 }
 
 // Backward: dq/dk (post-RoPE grads) -> grads w.r.t. the projection output (written into dqkv's q and
-// k column ranges) and partial weight grads accumulated with fp32 atomics into dqw/dkw [128].
+// k column ranges) and partial weight grads accumulated with fp32 atomics into dqw/dkw [128].  CTAs stay for several tokens and
+// end with one atomic per channel: a CTA per eight tokens whose lanes all added to shared memory with atomics (compare-and-swap
+// loops for floats) took 60 us for 8192 tokens of 16:8 heads, twice its traffic; now 42.
 __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(
     const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk,
     const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ qw,
@@ -465,9 +471,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(
     const float* __restrict__ cos_t, const float* __restrict__ sin_t,
     const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dqkv, float* __restrict__ dqw,
     float* __restrict__ dkw, int M, int Hq, int Hkv, int ld_qkv) {
-  __shared__ float sdw[2][128];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) (&sdw[0][0])[i] = 0.f;
-  __syncthreads();
+  __shared__ float sdw[8][2][128];
   const int heads = Hq + Hkv;
   const int lane = threadIdx.x & 31, l16 = lane & 15, sub = lane >> 4;
   const int warps_per_grid = (gridDim.x * blockDim.x) >> 5;
@@ -536,16 +540,21 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(
       }
     }
   }
+  // the two heads of a warp-wide access, the warps of the CTA (in order), then one atomic per channel and CTA
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    atomicAdd(&sdw[0][l16 * 8 + j], dwq[j]);
-    atomicAdd(&sdw[1][l16 * 8 + j], dwk[j]);
+    dwq[j] += __shfl_xor_sync(0xffffffffu, dwq[j], 16);
+    dwk[j] += __shfl_xor_sync(0xffffffffu, dwk[j], 16);
+    if (sub == 0) {
+      sdw[threadIdx.x >> 5][0][l16 * 8 + j] = dwq[j];
+      sdw[threadIdx.x >> 5][1][l16 * 8 + j] = dwk[j];
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) {
-    atomicAdd(dqw + i, sdw[0][i]);
-    atomicAdd(dkw + i, sdw[1][i]);
-  }
+  float t = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) t += sdw[k][threadIdx.x >> 7][threadIdx.x & 127];
+  atomicAdd((threadIdx.x >> 7 ? dkw : dqw) + (threadIdx.x & 127), t);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -656,42 +665,75 @@ B2_EXPORT int b2_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd,
   return 0;
 }
 
+// One launch of the row kernel; returns the number of CTAs (rows of dw_partial), or -1.  ctas: the most that may be used.
+template <int NV, bool DW>
+static int launch_rms_bwd_rows(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* partial, int M, int H,
+                               int add_to_dx, int ctas, cudaStream_t stream) {
+  auto kern = rmsnorm_bwd_rows_kernel<NV, DW>;
+  const int smem = DW ? 8 * H * static_cast<int>(sizeof(float)) : 0;
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (DW && !configured[dev & 63].load(std::memory_order_relaxed)) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 256 * NV * static_cast<int>(sizeof(float))) !=
+        cudaSuccess)
+      return -1;
+    configured[dev & 63].store(true, std::memory_order_relaxed);
+  }
+  if (ctas > (M + 7) / 8) ctas = (M + 7) / 8;
+  kern<<<ctas, 256, smem, stream>>>(static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+                                    static_cast<const __nv_bfloat16*>(w), rstd, static_cast<__nv_bfloat16*>(dx), partial, M, H, add_to_dx);
+  return ctas;
+}
+
 // dw_partial: fp32 scratch of at least b2_rmsnorm_bwd_ctas() * H floats.
 B2_EXPORT int b2_rmsnorm_bwd_ctas() {
   b2::ensure_thread_context(); return num_sms() * 2; }
 
+// dw == nullptr: the weight is frozen, only dx is computed (dw_partial is not used either).
 B2_EXPORT int b2_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
                              void* dw, float* dw_partial, int M, int H, int add_to_dx,
                              int accumulate_dw, int dw_fp32, void* stream_) {
   b2::ensure_thread_context();
-  if (H % 8 || H > RMS_THREADS * 8 * RMS_MAX_VEC) { set_error("rmsnorm_bwd: H must be a multiple of 8 and <= 8192"); return 10; }
+  if (H % 8 || H > RMS_THREADS * 8 * RMS_MAX_VEC || (dw == nullptr && H > 4096 && dw_partial == nullptr)) {
+    set_error("rmsnorm_bwd: H must be a multiple of 8 and <= 8192");
+    return 10;
+  }
   if (M <= 0) return 0;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   int ctas = num_sms() * 2;
-  if (ctas > M) ctas = M;
-  if (H <= 2048 && 256 % (H / 8) == 0) {
-    auto dys = static_cast<const __nv_bfloat16*>(dy);
-    auto xs = static_cast<const __nv_bfloat16*>(x);
-    auto ws = static_cast<const __nv_bfloat16*>(w);
-    auto dxs = static_cast<__nv_bfloat16*>(dx);
-    int blocks = (M + 7) / 8;
-    const int cap = num_sms() * 8;
-    if (blocks > cap) blocks = cap;
-    if (H <= 1024) rmsnorm_bwd_dx_kernel<4><<<blocks, 256, 0, stream>>>(dys, xs, ws, rstd, dxs, M, H, add_to_dx);
-    else rmsnorm_bwd_dx_kernel<8><<<blocks, 256, 0, stream>>>(dys, xs, ws, rstd, dxs, M, H, add_to_dx);
-    B2_LAUNCH_CHECK("rmsnorm_bwd_dx");
-    const int dw_ctas = ctas > num_sms() ? num_sms() : ctas;
-    rmsnorm_bwd_dw_kernel<<<dw_ctas, 256, H * static_cast<int>(sizeof(float)), stream>>>(dys, xs, rstd, dw_partial, M, H);
-    B2_LAUNCH_CHECK("rmsnorm_bwd_dw");
-    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(dw_partial, dw, dw_ctas, H, accumulate_dw, dw_fp32);
-    B2_LAUNCH_CHECK("rmsnorm_bwd_reduce");
-    return 0;
+  // Rows of up to 3072 columns with their column sums (4096 without) fit a warp's registers; two CTAs an SM, one from 2049
+  // columns on (about 220 registers a thread).  Longer rows take a CTA each.
+#define B2_RMS_ROWS(NV_, DW_, CTAS_) \
+  ctas = launch_rms_bwd_rows<NV_, DW_>(dy, x, w, rstd, dx, dw_partial, M, H, add_to_dx, CTAS_, stream)
+  const int sms = num_sms();
+  bool rows = true;
+  if (dw == nullptr) {
+    if (H <= 1024) B2_RMS_ROWS(4, false, sms * 8);
+    else if (H <= 2048) B2_RMS_ROWS(8, false, sms * 4);
+    else if (H <= 3072) B2_RMS_ROWS(12, false, sms * 2);
+    else if (H <= 4096) B2_RMS_ROWS(16, false, sms * 2);
+    else rows = false;
+  } else {
+    if (H <= 1024) B2_RMS_ROWS(4, true, sms * 2);
+    else if (H <= 2048) B2_RMS_ROWS(8, true, sms);
+    else if (H <= 3072) B2_RMS_ROWS(12, true, sms);
+    else rows = false;
   }
-  rmsnorm_bwd_kernel<<<ctas, RMS_THREADS, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
-      static_cast<const __nv_bfloat16*>(w), rstd, static_cast<__nv_bfloat16*>(dx), dw_partial, M, H,
-      add_to_dx);
+#undef B2_RMS_ROWS
+  if (!rows) {
+    if (ctas > M) ctas = M;
+    rmsnorm_bwd_kernel<<<ctas, RMS_THREADS, 0, stream>>>(
+        static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+        static_cast<const __nv_bfloat16*>(w), rstd, static_cast<__nv_bfloat16*>(dx), dw_partial, M, H,
+        add_to_dx);
+  }
+  if (ctas < 0) {
+    set_error("rmsnorm_bwd: cannot set the shared memory size");
+    return 1;
+  }
   B2_LAUNCH_CHECK("rmsnorm_bwd");
+  if (dw == nullptr) return 0;
   reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(dw_partial, dw, ctas, H, accumulate_dw, dw_fp32);
   B2_LAUNCH_CHECK("rmsnorm_bwd_reduce");
   return 0;
@@ -749,7 +791,7 @@ B2_EXPORT int b2_qknorm_rope_bwd(const void* dq, const void* dk, const void* qkv
   if (head_dim != 128) { set_error("qknorm_rope: head_dim must be 128"); return 10; }
   if (M <= 0) return 0;
   long long blocks = (static_cast<long long>(M) + 7) / 8;   // one warp per token
-  const long long cap = static_cast<long long>(num_sms()) * 8;
+  const long long cap = static_cast<long long>(num_sms()) * QKB_CTAS;
   if (blocks > cap) blocks = cap;
   qknorm_rope_bwd_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dq), static_cast<const __nv_bfloat16*>(dk),
@@ -861,20 +903,14 @@ B2_EXPORT int b2_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* 
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   int dw_ctas = num_sms();
   if (dw_ctas > B2_NOALLOC_MAX_PARTIALS) dw_ctas = B2_NOALLOC_MAX_PARTIALS;
-  if (dw_ctas > M) dw_ctas = M;
-  auto dys = static_cast<const __nv_bfloat16*>(dy);
-  auto xs = static_cast<const __nv_bfloat16*>(x);
-  auto ws = static_cast<const __nv_bfloat16*>(w);
-  auto dxs = static_cast<__nv_bfloat16*>(dx);
-  int blocks = (M + 7) / 8;
-  const int cap = num_sms() * 8;
-  if (blocks > cap) blocks = cap;
-  if (H <= 1024) rmsnorm_bwd_dx_kernel<4><<<blocks, 256, 0, stream>>>(dys, xs, ws, rstd, dxs, M, H, add_to_dx);
-  else rmsnorm_bwd_dx_kernel<8><<<blocks, 256, 0, stream>>>(dys, xs, ws, rstd, dxs, M, H, add_to_dx);
-  B2_LAUNCH_CHECK("rmsnorm_bwd_noalloc(dx)");
   // every CTA writes its whole [H] row of partials, so stale contents of the shared array are never read
-  rmsnorm_bwd_dw_kernel<<<dw_ctas, 256, H * static_cast<int>(sizeof(float)), stream>>>(dys, xs, rstd, partial, M, H);
-  B2_LAUNCH_CHECK("rmsnorm_bwd_noalloc(dw)");
+  dw_ctas = H <= 1024 ? launch_rms_bwd_rows<4, true>(dy, x, w, rstd, dx, partial, M, H, add_to_dx, dw_ctas, stream)
+                      : launch_rms_bwd_rows<8, true>(dy, x, w, rstd, dx, partial, M, H, add_to_dx, dw_ctas, stream);
+  if (dw_ctas < 0) {
+    set_error("rmsnorm_bwd_noalloc: cannot set the shared memory size");
+    return 1;
+  }
+  B2_LAUNCH_CHECK("rmsnorm_bwd_noalloc");
   reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(partial, dw, dw_ctas, H, accumulate_dw, dw_fp32);
   B2_LAUNCH_CHECK("rmsnorm_bwd_noalloc(reduce)");
   return 0;

@@ -125,3 +125,41 @@ def test_products_with_few_rows_take_every_epilogue(act, M):
     got, floor = _error(gemm(a, b, bn=128), prod)       # a given width keeps the persistent kernel
     assert got <= 1.02 * floor + 1e-5
     assert torch.equal(gemm(a, b), gemm(a, b))
+
+
+@pytest.mark.parametrize("M,H", [(1, 1024), (7, 256), (2500, 1000), (300, 2048), (2400, 2560), (33, 3072), (40, 3080), (50, 4096), (20, 5120)])
+@pytest.mark.parametrize("frozen", [False, True])
+def test_rmsnorm_backward_over_row_lengths(M, H, frozen):
+    """Row lengths on either side of each register layout, whole and ragged warps, a frozen weight (no column sums)."""
+    from b200fw.ops import rmsnorm
+    g = torch.Generator(device=DEV).manual_seed(6)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    x, w, dy = rnd(M, H).to(torch.bfloat16).requires_grad_(), (1 + 0.1 * rnd(H)).to(torch.bfloat16), rnd(M, H).to(torch.bfloat16)
+    w.requires_grad_(not frozen)
+    rmsnorm(x, w).backward(dy)
+    xd, wd = x.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    (xd * torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-6) * wd).backward(dy.double())
+    got, floor = _error(x.grad, xd.grad)
+    assert got <= 1.02 * floor + 1e-5, (got, floor)       # 32-bit arithmetic on the way to a bf16 result
+    if frozen:
+        assert w.grad is None
+    else:
+        got, floor = _error(w.grad, wd.grad)
+        assert got <= 1.02 * floor + 1e-5, (got, floor)
+
+
+def test_attention_backward_of_ragged_rows():
+    """231 rows of dO * O: the last warp of the row sums is not full."""
+    from b200fw.ops import flash_attention
+    g = torch.Generator(device=DEV).manual_seed(7)
+    B, S, Hq, Hkv = 1, 77, 3, 1
+    q, k, v = (torch.randn(B * S, h * 128, device=DEV, generator=g).to(torch.bfloat16).requires_grad_() for h in (Hq, Hkv, Hkv))
+    dy = torch.randn(B * S, Hq * 128, device=DEV, generator=g).to(torch.bfloat16)
+    flash_attention(q, k, v, B, S, Hq, Hkv).backward(dy)
+    qd, kd, vd = (t.detach().double().requires_grad_() for t in (q, k, v))
+    s = torch.einsum("qhd,kd->hqk", qd.reshape(S, Hq, 128), kd) / math.sqrt(128)
+    s = s.masked_fill(torch.ones(S, S, device=DEV, dtype=torch.bool).triu(1), -math.inf).softmax(-1)
+    torch.einsum("hqk,kd->qhd", s, vd).reshape(S, -1).backward(dy.double())
+    for a, b in ((q, qd), (k, kd), (v, vd)):
+        # P and dS are bf16 operands of the gradient products: 2^-9 each, a few of them added up
+        assert _error(a.grad, b.grad)[0] < 1e-2
