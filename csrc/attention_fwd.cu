@@ -673,391 +673,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
-// ---------------------------------------------------------------------------------------------------------------------
-// Plain causal form (head size 128, no options).  A CTA works on TWO query tiles over the same keys: two query heads of one kv head,
-// or, where the heads do not pair up, two neighbouring query tiles of one head.
-//
-// A 128 x 128 tile costs 1024 cycles of MMA and 1024 of the special-function unit (16 exponentials a cycle), so the two have to
-// overlap.  With one query tile at a time every softmax warp does the same thing at the same time: while it reads scores, finds
-// maxima or waits, neither unit works (2650 cycles a tile on long sequences, 4000 on prompt chunks).  Here the tiles take
-// turns: while the softmax of one runs, the tensor cores do the other's P V and next Q K^T, and each K / V tile is
-// loaded once for both.  A thread owns a whole row, so no exchange between threads is left.  8 x 1024 tokens, 16:8 heads: 73 ->
-// 63 us; chunks of 2048 of a paged 8192-token prompt: 115 -> 105 us on average.
-//
-// Roles (FP_THREADS = 320): warp 0 TMA, warp 1 issues all MMAs, warps 2..5 softmax of tile 0, warps 6..9 of tile 1.
-// TMEM: S of the two tiles 2 x 128 columns, O 2 x 128; P (bf16 pairs) overwrites the front of its own S.  The MMA warp's order,
-// PV_0(j) QK_0(j+1) PV_1(j) QK_1(j+1), is what makes that safe: QK_g(j+1) is issued after PV_g(j), PV_g(j) after P_g(j) was
-// written, and MMAs complete in order, so s_full also says that the previous P V is in O.  The next item's first Q K^T is
-// issued by the same order, before the last item's write-out.
-// ---------------------------------------------------------------------------------------------------------------------
-constexpr int FP_THREADS = 320;
-struct AttnPairSmem {
-  static constexpr int Q = 0;                           // one tile per group
-  static constexpr int K = Q + 2 * AT_TILE_BYTES;       // 2 stages
-  static constexpr int V = K + 2 * AT_TILE_BYTES;       // 2 stages
-  static constexpr int EPI = V + 2 * AT_TILE_BYTES;     // 8 warps x 4 KiB write-out staging
-  static constexpr int BARS = EPI + 8 * 4096;
-  static constexpr int TOTAL = BARS + 256 + 1024;
-  static_assert(TOTAL <= 232448, "shared memory of one CTA");
-};
-
-struct PairItem {
-  int head[2], qt[2], n[2];     // n: key tiles of each group's query tile (0: no tile)
-  int n_kv, kvh, batch, q_begin, q_len, kv_len, kv_off, k_begin;
-};
-__device__ __forceinline__ bool pair_item(int w, const FwdParams& p, PairItem& it) {
-  const bool heads = (p.Hq / p.Hkv) % 2 == 0;
-  const int units = heads ? p.Hq / 2 : p.Hq;
-  const int hb = w % (units * p.B), x = w / (units * p.B);   // x: rank counted from the last (heaviest) tile
-  const int unit = hb % units;
-  it.batch = hb / units;
-  it.q_begin = p.cu_q ? p.cu_q[it.batch] : it.batch * p.S;
-  it.q_len = p.cu_q ? p.cu_q[it.batch + 1] - it.q_begin : p.S;
-  it.k_begin = p.cu_k ? p.cu_k[it.batch] : it.batch * p.S;
-  it.kv_len = p.cu_k ? p.cu_k[it.batch + 1] - it.k_begin : p.S;
-  it.kv_off = it.kv_len - it.q_len;
-  const int tiles = (it.q_len + 127) / 128;
-  it.n_kv = 0;
-#pragma unroll
-  for (int g = 0; g < 2; ++g) {
-    it.head[g] = heads ? 2 * unit + g : unit;
-    it.qt[g] = heads ? tiles - 1 - x : 2 * ((tiles + 1) / 2 - 1 - x) + g;
-    const bool live = it.q_len > 0 && it.qt[g] >= 0 && it.qt[g] < tiles;
-    it.n[g] = live ? (min(it.kv_len, it.kv_off + (it.qt[g] + 1) * 128) + 127) / 128 : 0;
-    it.n_kv = max(it.n_kv, it.n[g]);
-  }
-  it.kvh = it.head[0] / (p.Hq / p.Hkv);
-  return it.n_kv > 0;
-}
-__device__ __forceinline__ int pair_first(int n_items, const FwdParams& p, PairItem& it) {
-  int w = blockIdx.x;
-  while (w < n_items && !pair_item(w, p, it)) w = snake_next(w);
-  return w;
-}
-__device__ __forceinline__ int pair_next(int w, int n_items, const FwdParams& p, PairItem& it) {
-  w = snake_next(w);
-  while (w < n_items && !pair_item(w, p, it)) w = snake_next(w);
-  return w;
-}
-
-__global__ void __launch_bounds__(FP_THREADS, 1)
-attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ out,
-                     float* __restrict__ lse_out, const FwdParams prm, int n_items, float scale, int* status) {
-  using Smem = AttnPairSmem;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Smem::BARS);
-  uint64_t *q_full = bars, *q_empty = bars + 2, *k_full = bars + 4, *k_empty = bars + 6, *v_full = bars + 8, *v_empty = bars + 10,
-           *s_full = bars + 12, *p_full = bars + 14, *o_done = bars + 16, *o_free = bars + 18;     // two each
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int Hq = prm.Hq;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&q_full[i], 1);
-      mbar_init(&q_empty[i], 1);
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 4);     // one arrive per softmax warp of the group
-      mbar_init(&o_done[i], 1);
-      mbar_init(&o_free[i], 4);
-    }
-    mbar_fence_init();
-    tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_S = *reinterpret_cast<volatile uint32_t*>(tmem_slot);   // group g: S (and P) at + 128 g
-  const uint32_t tmem_O = tmem_S + 256;                                       // O at + 128 g
-  PairItem it;
-  int w = pair_first(n_items, prm, it);
-
-  if (warp == 0) {
-    if (lane == 0) {
-      int g = 0, nq[2] = {0, 0};     // key tiles so far; items so far per group
-      bool ok = true;
-      // one [128 x 128] tile of keys or values
-      auto load_kv = [&](const CUtensorMap* map, uint8_t* dst, uint64_t* bar, int j) {
-        mbar_expect_tx(bar, AT_TILE_BYTES);
-        if (prm.block_tables != nullptr) {
-          // eight 16-token pages: each lands as a [16 x 64] box at its row offset of the swizzled tile (16 rows x 128 B =
-          // 2 KiB, a whole number of swizzle atoms).  Pages past the end of the sequence repeat its last page: those keys
-          // are masked, the bytes only have to be finite.
-          const int* tbl = prm.block_tables + static_cast<size_t>(it.batch) * prm.max_blocks;
-          const int last_page = (it.kv_len - 1) / 16;
-          int rows[8];
-#pragma unroll
-          for (int pg = 0; pg < 8; ++pg) rows[pg] = tbl[min(j * 8 + pg, last_page)] * 16;
-#pragma unroll
-          for (int pg = 0; pg < 8; ++pg) {
-            tma_load_2d(dst + pg * 2048, map, bar, it.kvh * 128, rows[pg]);
-            tma_load_2d(dst + AT_HALF_BYTES + pg * 2048, map, bar, it.kvh * 128 + 64, rows[pg]);
-          }
-        } else {
-          tma_load_2d(dst, map, bar, it.kvh * 128, it.k_begin + j * 128);
-          tma_load_2d(dst + AT_HALF_BYTES, map, bar, it.kvh * 128 + 64, it.k_begin + j * 128);
-        }
-      };
-      for (; w < n_items && ok; w = pair_next(w, n_items, prm, it)) {
-        for (int j = 0; j < it.n_kv && ok; ++j, ++g) {
-          const int st = g & 1;
-          const uint32_t ph = (g >> 1) & 1;
-          if (!mbar_wait(&k_empty[st], ph ^ 1, status, ERR_ATTN_WAIT)) { ok = false; break; }
-          load_kv(&tmK, smem + Smem::K + st * AT_TILE_BYTES, &k_full[st], j);
-          if (j == 0) {
-            for (int x = 0; x < 2; ++x) {
-              if (it.n[x] == 0) continue;
-              if (!mbar_wait(&q_empty[x], (nq[x] & 1) ^ 1, status, ERR_ATTN_WAIT)) { ok = false; break; }
-              ++nq[x];
-              uint8_t* sQ = smem + Smem::Q + x * AT_TILE_BYTES;
-              mbar_expect_tx(&q_full[x], AT_TILE_BYTES);
-              tma_load_2d(sQ, &tmQ, &q_full[x], it.head[x] * 128, it.q_begin + it.qt[x] * 128);
-              tma_load_2d(sQ + AT_HALF_BYTES, &tmQ, &q_full[x], it.head[x] * 128 + 64, it.q_begin + it.qt[x] * 128);
-            }
-            if (!ok) break;
-          }
-          if (!mbar_wait(&v_empty[st], ph ^ 1, status, ERR_ATTN_WAIT)) { ok = false; break; }
-          load_kv(&tmV, smem + Smem::V + st * AT_TILE_BYTES, &v_full[st], j);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    const bool leader = elect_one();
-    constexpr uint32_t idesc_s = make_idesc_f16(1, 128, 128, 0, 0), idesc_pv = make_idesc_f16(1, 128, 128, 0, 1);
-    int kg = 0, vg = 0, nq[2] = {0, 0}, np[2] = {0, 0}, no[2] = {0, 0};   // tiles; per group: items begun, P tiles, items ended
-    bool ok = true;
-    auto qk = [&](int x, int n, int j) {     // S_x of key tile j of an item whose group x has n tiles; K is in stage kg & 1
-      if (j >= n || !ok) return;
-      if (j == 0) {
-        if (!mbar_wait(&q_full[x], nq[x] & 1, status, ERR_ATTN_WAIT)) { ok = false; return; }
-        ++nq[x];
-      }
-      tc_fence_after();
-      const uint64_t d_q = make_smem_desc_sw128(smem_u32(smem + Smem::Q + x * AT_TILE_BYTES), 16, 1024);
-      const uint64_t d_k = make_smem_desc_sw128(smem_u32(smem + Smem::K + (kg & 1) * AT_TILE_BYTES), 16, 1024);
-      if (leader) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t o = (ks >> 2) * AT_HALF_BYTES + (ks & 3) * 32;
-          umma_f16_ss(tmem_S + x * 128, desc_advance(d_q, o), desc_advance(d_k, o), idesc_s, ks != 0);
-        }
-        umma_commit(&s_full[x]);
-        if (j + 1 == n) umma_commit(&q_empty[x]);
-      }
-    };
-    auto pv = [&](int x, int n, int j) {
-      if (j >= n || !ok) return;
-      if (!mbar_wait(&p_full[x], np[x] & 1, status, ERR_ATTN_WAIT) ||
-          (j == 0 && no[x] > 0 && !mbar_wait(&o_free[x], (no[x] - 1) & 1, status, ERR_ATTN_WAIT)) ||
-          !mbar_wait(&v_full[vg & 1], (vg >> 1) & 1, status, ERR_ATTN_WAIT)) {
-        ok = false;
-        return;
-      }
-      ++np[x];
-      tc_fence_after();
-      const uint64_t d_v = make_smem_desc_sw128(smem_u32(smem + Smem::V + (vg & 1) * AT_TILE_BYTES), AT_HALF_BYTES, 1024);
-      const uint32_t acc0 = j != 0;
-      if (leader) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)   // A = P from TMEM: 16 bf16 of K per instruction = 8 columns
-          umma_f16_ts(tmem_O + x * 128, tmem_S + x * 128 + ks * 8, desc_advance(d_v, ks * 2048), idesc_pv, ks ? 1u : acc0);
-        if (j + 1 == n) umma_commit(&o_done[x]);
-      }
-      if (j + 1 == n) ++no[x];
-    };
-    auto wait_k = [&]() {
-      if (ok && !mbar_wait(&k_full[kg & 1], (kg >> 1) & 1, status, ERR_ATTN_WAIT)) ok = false;
-    };
-    if (w < n_items) {
-      wait_k();
-      qk(0, it.n[0], 0);
-      qk(1, it.n[1], 0);
-      if (leader && ok) umma_commit(&k_empty[kg & 1]);
-      ++kg;
-    }
-    int j = 0;
-    while (w < n_items && ok) {
-      const int n0 = it.n[0], n1 = it.n[1], jc = j;
-      if (++j == it.n_kv) {      // the step after this one belongs to the next item
-        w = pair_next(w, n_items, prm, it);
-        j = 0;
-      }
-      const bool more = w < n_items;
-      pv(0, n0, jc);
-      if (more) {
-        wait_k();
-        qk(0, it.n[0], j);
-      }
-      pv(1, n1, jc);
-      if (leader && ok) umma_commit(&v_empty[vg & 1]);
-      ++vg;
-      if (more) {
-        qk(1, it.n[1], j);
-        if (leader && ok) umma_commit(&k_empty[kg & 1]);
-        ++kg;
-      }
-    }
-  } else {
-    const int grp = (warp - 2) >> 2, quarter = warp & 3;
-    const int r = quarter * 32 + lane;        // query row inside the tile
-    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t tS = tmem_S + lane_off + grp * 128, tO = tmem_O + lane_off + grp * 128;
-    const float sl2 = scale * 1.4426950408889634f;
-    const float2 sl2_2 = make_float2(sl2, sl2), one2 = make_float2(1.f, 1.f);
-    uint8_t* stage = smem + Smem::EPI + (warp - 2) * 4096;
-    int ns = 0, no = 0;       // tiles and items of this group so far
-    bool ok = true;
-    for (; w < n_items && ok; w = pair_next(w, n_items, prm, it)) {
-      const int n = grp ? it.n[1] : it.n[0], qt = grp ? it.qt[1] : it.qt[0], head = grp ? it.head[1] : it.head[0];
-      if (n == 0) continue;
-      const int q_idx = qt * 128 + r, q_pos = it.kv_off + q_idx;    // index among the sequence's queries; last key it may see
-      float m_used = -INFINITY, l = 0.f;
-      for (int j = 0; j < n; ++j, ++ns) {
-        if (!mbar_wait_warp(&s_full[grp], ns & 1, status, ERR_ATTN_WAIT)) { ok = false; break; }
-        tc_fence_after();
-        float s[128];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(tS + c * 32, reinterpret_cast<uint32_t(&)[32]>(s[c * 32]));
-        tmem_ld_wait();
-        if ((j + 1) * 128 > it.kv_off + qt * 128 + 1 || (j + 1) * 128 > it.kv_len) {
-          const int last = min(q_pos, it.kv_len - 1) - j * 128;
-#pragma unroll
-          for (int i = 0; i < 128; ++i)
-            if (i > last) s[i] = -INFINITY;
-        }
-        float mx0 = s[0], mx1 = s[1], mx2 = s[2], mx3 = s[3];
-#pragma unroll
-        for (int i = 4; i < 128; i += 4) {
-          mx0 = fmaxf(mx0, s[i]);
-          mx1 = fmaxf(mx1, s[i + 1]);
-          mx2 = fmaxf(mx2, s[i + 2]);
-          mx3 = fmaxf(mx3, s[i + 3]);
-        }
-        const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)));
-        if (j > 0) {
-          const bool need = (m_new - m_used) * sl2 > 8.f;
-          if (__any_sync(0xffffffffu, need)) {   // rare: O (complete up to the last tile, see s_full) is rescaled
-            const float alpha = need ? exp2f((m_used - m_new) * sl2) : 1.f;
-#pragma unroll 1
-            for (int c = 0; c < 8; ++c) {
-              uint32_t t[16];
-              tmem_ld_32x32b_x16(tO + c * 16, t);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 16; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-              tmem_st_32x32b_x16(tO + c * 16, t);
-            }
-            if (need) {
-              l *= alpha;
-              m_used = m_new;
-            }
-          }
-        } else {
-          m_used = m_new;
-        }
-        const float2 mb2 = make_float2(-m_used * sl2, -m_used * sl2);
-        float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t pk[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float2 t = fma_f32x2(make_float2(s[c * 16 + 2 * i], s[c * 16 + 2 * i + 1]), sl2_2, mb2);
-            const float2 p = make_float2(fast_exp2(t.x), fast_exp2(t.y));
-            if (i & 1) sum1 = fma_f32x2(p, one2, sum1);
-            else sum0 = fma_f32x2(p, one2, sum0);
-            pk[i] = pack_bf16x2(p.x, p.y);
-          }
-          tmem_st_32x32b_x8(tS + c * 8, pk);
-        }
-        tmem_st_wait();
-        l += (sum0.x + sum0.y) + (sum1.x + sum1.y);
-        tc_fence_before();
-        mbar_arrive_warp(&p_full[grp]);
-      }
-      if (!ok || !mbar_wait_warp(&o_done[grp], no & 1, status, ERR_ATTN_WAIT)) { ok = false; break; }
-      ++no;
-      tc_fence_after();
-      const float inv = 1.f / l;
-      const int wq0 = qt * 128 + quarter * 32;   // index (within the sequence) of this warp's first query row
-      __nv_bfloat16* base = out + (static_cast<size_t>(it.q_begin + wq0) * Hq + head) * 128;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint4 ov[8];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t t[32];
-          tmem_ld_32x32b_x32(tO + h * 64 + c * 32, t);
-          tmem_ld_wait();
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            ov[c * 4 + v].x = pack_bf16x2(__uint_as_float(t[v * 8 + 0]) * inv, __uint_as_float(t[v * 8 + 1]) * inv);
-            ov[c * 4 + v].y = pack_bf16x2(__uint_as_float(t[v * 8 + 2]) * inv, __uint_as_float(t[v * 8 + 3]) * inv);
-            ov[c * 4 + v].z = pack_bf16x2(__uint_as_float(t[v * 8 + 4]) * inv, __uint_as_float(t[v * 8 + 5]) * inv);
-            ov[c * 4 + v].w = pack_bf16x2(__uint_as_float(t[v * 8 + 6]) * inv, __uint_as_float(t[v * 8 + 7]) * inv);
-          }
-        }
-        if (h == 1) {
-          tc_fence_before();
-          mbar_arrive_warp(&o_free[grp]);   // this warp's part of O is in registers
-        }
-        warp_store_rows_128B(stage, ov, [&](int row) -> uint8_t* {
-          if (wq0 + row >= it.q_len) return nullptr;
-          return reinterpret_cast<uint8_t*>(base + static_cast<size_t>(row) * Hq * 128 + h * 64);
-        });
-      }
-      if (q_idx < it.q_len && lse_out)
-        lse_out[static_cast<size_t>(head) * prm.total_q + it.q_begin + q_idx] = m_used * scale + __logf(l);
-    }
-  }
-
-  if (*reinterpret_cast<volatile int*>(status) != 0) {
-    unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    __syncwarp();
-    tc_fence_after();
-    tmem_dealloc(tmem_S, 512);
-  }
-}
-
-static int launch_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* out, float* lse, const FwdParams& prm,
-                       float scale, int* status, cudaStream_t stream) {
-  static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!configured[dev]) {
-    if (cudaFuncSetAttribute(attn_fwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnPairSmem::TOTAL) != cudaSuccess) {
-      set_error("attn_fwd: cannot set shared memory size");
-      return 1;
-    }
-    configured[dev] = true;
-  }
-  const bool heads = (prm.Hq / prm.Hkv) % 2 == 0;
-  const long long n_items = static_cast<long long>(heads ? prm.max_tiles : (prm.max_tiles + 1) / 2) * (heads ? prm.Hq / 2 : prm.Hq) * prm.B;
-  const int grid = n_items < num_sms() ? static_cast<int>(n_items) : num_sms();
-  attn_fwd_pair_kernel<<<grid, FP_THREADS, AttnPairSmem::TOTAL, stream>>>(tq, tk, tv, static_cast<__nv_bfloat16*>(out), lse, prm,
-                                                                          static_cast<int>(n_items), scale, status);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_error("attn_fwd launch failed: %s", cudaGetErrorString(e));
-    return 4;
-  }
-  return 0;
+static FwdExt no_ext() {
+  FwdExt e = {};
+  e.maps = 1;
+  return e;
 }
 
 }  // namespace b2
@@ -1089,6 +708,17 @@ B2_EXPORT int b2_attn_fwd_varlen(const void* q, const void* k, const void* v, vo
   }
   if (B <= 0 || max_q <= 0 || total_q <= 0) return 0;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(attn_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             AttnFwdSmem::TOTAL) != cudaSuccess) {
+      set_error("attn_fwd: cannot set shared memory size");
+      return 1;
+    }
+    configured[dev] = true;
+  }
   const CUtensorMap* tq = tensor_map_2d_bf16(q, total_q, static_cast<uint64_t>(Hq) * 128, static_cast<uint64_t>(Hq) * 128, 128, 64);
   const CUtensorMap* tk = tensor_map_2d_bf16(k, total_k, static_cast<uint64_t>(Hkv) * 128, ld_k, 128, 64);
   const CUtensorMap* tv = tensor_map_2d_bf16(v, total_k, static_cast<uint64_t>(Hkv) * 128, ld_v, 128, 64);
@@ -1099,7 +729,16 @@ B2_EXPORT int b2_attn_fwd_varlen(const void* q, const void* k, const void* v, vo
   prm.S = S; prm.Hq = Hq; prm.Hkv = Hkv; prm.B = B; prm.max_tiles = (max_q + 127) / 128; prm.total_q = total_q;
   prm.cu_q = cu_q; prm.cu_k = cu_k;
   prm.block_tables = nullptr; prm.max_blocks = 0;
-  return launch_pair(*tq, *tk, *tv, out, lse, prm, scale, status, stream);
+  const long long n_items = static_cast<long long>(prm.max_tiles) * Hq * B;
+  const int grid = n_items < num_sms() ? static_cast<int>(n_items) : num_sms();
+  attn_fwd_kernel<false><<<grid, AT_THREADS, AttnFwdSmem::TOTAL, stream>>>(
+      *tq, *tk, *tv, static_cast<__nv_bfloat16*>(out), lse, prm, no_ext(), scale, status);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error("attn_fwd launch failed: %s", cudaGetErrorString(e));
+    return 4;
+  }
+  return 0;
 }
 
 // Chunked prefill over the paged KV cache: the keys / values of sequence b are the first kv_len[b] tokens of the
@@ -1117,6 +756,17 @@ B2_EXPORT int b2_attn_fwd_paged(const void* q, const void* k_cache, const void* 
   }
   if (B <= 0 || max_q <= 0 || total_q <= 0) return 0;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(attn_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             AttnFwdSmem::TOTAL) != cudaSuccess) {
+      set_error("attn_fwd_paged: cannot set shared memory size");
+      return 1;
+    }
+    configured[dev] = true;
+  }
   const uint64_t W = static_cast<uint64_t>(Hkv) * 128;
   const CUtensorMap* tq = tensor_map_2d_bf16(q, total_q, static_cast<uint64_t>(Hq) * 128, static_cast<uint64_t>(Hq) * 128, 128, 64);
   const CUtensorMap* tk = tensor_map_2d_bf16(k_cache, static_cast<uint64_t>(num_blocks) * 16, W, W, 16, 64);
@@ -1128,7 +778,16 @@ B2_EXPORT int b2_attn_fwd_paged(const void* q, const void* k_cache, const void* 
   prm.S = 0; prm.Hq = Hq; prm.Hkv = Hkv; prm.B = B; prm.max_tiles = (max_q + 127) / 128; prm.total_q = total_q;
   prm.cu_q = cu_q; prm.cu_k = cu_k;
   prm.block_tables = block_tables; prm.max_blocks = max_blocks;
-  return launch_pair(*tq, *tk, *tv, out, lse, prm, scale, status, stream);
+  const long long n_items = static_cast<long long>(prm.max_tiles) * Hq * B;
+  const int grid = n_items < num_sms() ? static_cast<int>(n_items) : num_sms();
+  attn_fwd_kernel<false><<<grid, AT_THREADS, AttnFwdSmem::TOTAL, stream>>>(
+      *tq, *tk, *tv, static_cast<__nv_bfloat16*>(out), lse, prm, no_ext(), scale, status);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error("attn_fwd_paged launch failed: %s", cudaGetErrorString(e));
+    return 4;
+  }
+  return 0;
 }
 
 // The extended form over the paged cache (see FwdExt): q [total_q, Hq * dkp], K pages [blocks, 16, Hkv, dkp], V pages
