@@ -149,6 +149,15 @@ __device__ __forceinline__ int snake_next(int w) {
   return (w / G + 1) * G + (G - 1 - w % G);
 }
 
+// ---- chained launches ----------------------------------------------------------------------------
+// A kernel launched with launch_chained (host.h) may start while the kernel before it in the stream still runs.  chain_wait
+// returns once that kernel is complete and its writes are visible: nothing that an earlier kernel may write is read, and
+// nothing that it may read is written, before it.  chain_release lets the next chained kernel start; it is given once this
+// CTA is short of finishing, so that the next kernel's CTAs do not sit on registers that other streams could use.  Both do nothing
+// in a kernel that was launched, or is followed, in the ordinary way.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- TMA ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");

@@ -43,4 +43,36 @@ inline int num_sms() {
   return n[dev];
 }
 
+// Steps of few rows (decoding, single short examples) are chains of short kernels: the launch, barrier set-up and first copies
+// of each are a large part of its time.  Up to this many rows a kernel is launched so that it may start before its
+// predecessor has ended (see chain_wait).  Larger ones run long enough to hide it, and keep the ordinary order of
+// launches, in which CTAs of one kernel never wait on an SM while another stream's kernel could use it.
+constexpr int CHAIN_ROWS = 512;
+
+// chained: allow the overlap described above; the kernel has to call chain_wait.  cluster_x, cluster_z: cluster shape (1: none).
+template <typename... P, typename... A>
+cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster_x,
+                           int cluster_z, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster_x * cluster_z > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster_x;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = cluster_z;
+  }
+  if (chained) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 }  // namespace b2

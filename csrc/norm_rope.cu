@@ -60,6 +60,8 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
     __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float scratch[32];
+  chain_wait();
+  chain_release();
   const size_t row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * H;
   __nv_bfloat16* yr = y + row * H;
@@ -184,6 +186,8 @@ template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
     __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int M, int H, float eps) {
+  chain_wait();
+  chain_release();
   const int lane = threadIdx.x & 31;
   const int warps_per_grid = (gridDim.x * blockDim.x) >> 5;
   const int nvec = H / 8;
@@ -394,6 +398,8 @@ __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(
     __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_out,
     float* __restrict__ rstd_out, int M, int Hq, int Hkv, int ld_qkv, float eps,
     const int* __restrict__ slots, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache) {
+  chain_wait();
+  chain_release();
   const int heads = Hq + Hkv;
   const int lane = threadIdx.x & 31, l16 = lane & 15, sub = lane >> 4;
   const int warps_per_grid = (gridDim.x * blockDim.x) >> 5;
@@ -562,6 +568,8 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(
 // ---------------------------------------------------------------------------------------------
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                   long long M, int I) {
+  chain_wait();
+  chain_release();
   const int nvec = I / 8;
   const long long total = M * nvec;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -653,12 +661,12 @@ B2_EXPORT int b2_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd,
     auto ws = static_cast<const __nv_bfloat16*>(w);
     auto ys = static_cast<__nv_bfloat16*>(y);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (H <= 1024) rmsnorm_fwd_warp_kernel<4><<<blocks, 256, 0, st>>>(xs, ws, ys, rstd, M, H, eps);
-    else rmsnorm_fwd_warp_kernel<8><<<blocks, 256, 0, st>>>(xs, ws, ys, rstd, M, H, eps);
+    if (H <= 1024) launch_chained(M <= CHAIN_ROWS, rmsnorm_fwd_warp_kernel<4>, dim3(blocks), 256, 0, st, 1, 1, xs, ws, ys, rstd, M, H, eps);
+    else launch_chained(M <= CHAIN_ROWS, rmsnorm_fwd_warp_kernel<8>, dim3(blocks), 256, 0, st, 1, 1, xs, ws, ys, rstd, M, H, eps);
     B2_LAUNCH_CHECK("rmsnorm_fwd");
     return 0;
   }
-  rmsnorm_fwd_kernel<<<M, RMS_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_chained(M <= CHAIN_ROWS, rmsnorm_fwd_kernel, dim3(M), RMS_THREADS, 0, static_cast<cudaStream_t>(stream), 1, 1,
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
       static_cast<__nv_bfloat16*>(y), rstd, H, eps);
   B2_LAUNCH_CHECK("rmsnorm_fwd");
@@ -749,7 +757,7 @@ B2_EXPORT int b2_qknorm_rope_fwd(const void* qkv, const void* qw, const void* kw
   long long blocks = (static_cast<long long>(M) + 7) / 8;   // one warp per token
   const long long fcap = static_cast<long long>(num_sms()) * 16;
   if (blocks > fcap) blocks = fcap;
-  qknorm_rope_fwd_kernel<false><<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_chained(M <= CHAIN_ROWS, qknorm_rope_fwd_kernel<false>, dim3(static_cast<unsigned>(blocks)), 256, 0, static_cast<cudaStream_t>(stream), 1, 1,
       static_cast<const __nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(qw),
       static_cast<const __nv_bfloat16*>(kw), pos, cos_t, sin_t, static_cast<__nv_bfloat16*>(q_out),
       static_cast<__nv_bfloat16*>(k_out), rstd, M, Hq, Hkv, ld_qkv, eps, nullptr, nullptr, nullptr);
@@ -773,7 +781,7 @@ B2_EXPORT int b2_qknorm_rope_store(const void* qkv, const void* qw, const void* 
   long long blocks = (static_cast<long long>(M) + 7) / 8;   // one warp per token
   const long long fcap = static_cast<long long>(num_sms()) * 16;
   if (blocks > fcap) blocks = fcap;
-  qknorm_rope_fwd_kernel<true><<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_chained(M <= CHAIN_ROWS, qknorm_rope_fwd_kernel<true>, dim3(static_cast<unsigned>(blocks)), 256, 0, static_cast<cudaStream_t>(stream), 1, 1,
       static_cast<const __nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(qw),
       static_cast<const __nv_bfloat16*>(kw), pos, cos_t, sin_t, static_cast<__nv_bfloat16*>(q_out),
       static_cast<__nv_bfloat16*>(k_out), nullptr, M, Hq, Hkv, ld_qkv, eps, slots,
@@ -810,7 +818,7 @@ B2_EXPORT int b2_swiglu_fwd(const void* gu, void* out, long long M, int I, void*
   long long blocks = (total + 255) / 256;
   const long long cap = static_cast<long long>(num_sms()) * 16;
   if (blocks > cap) blocks = cap;
-  swiglu_fwd_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_chained(M <= CHAIN_ROWS, swiglu_fwd_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, static_cast<cudaStream_t>(stream), 1, 1,
       static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), M, I);
   B2_LAUNCH_CHECK("swiglu_fwd");
   return 0;

@@ -38,6 +38,8 @@ __global__ void __launch_bounds__(128) kv_store_kernel(
     void* __restrict__ k_cache, void* __restrict__ v_cache, float* __restrict__ k_scale,
     float* __restrict__ v_scale, const int* __restrict__ segs, int Hkv) {
   __shared__ float red[4];
+  chain_wait();
+  chain_release();
   const int seg = blockIdx.x, h = blockIdx.y, which = blockIdx.z;
   const int block = segs[seg * 4 + 0], tok0 = segs[seg * 4 + 1], count = segs[seg * 4 + 2],
             off = segs[seg * 4 + 3];
@@ -437,6 +439,7 @@ __global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
     }
     __syncwarp();   // every lane has read the stage before its next copies are issued
   }
+  chain_release();
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncwarp();
 
@@ -562,11 +565,11 @@ B2_EXPORT int b2_kv_store(const void* k, const void* v, int ld_k, int ld_v, void
   if (nseg <= 0) return 0;
   dim3 grid(nseg, Hkv, 2);
   if (fp8)
-    kv_store_kernel<true><<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(nseg <= CHAIN_ROWS, kv_store_kernel<true>, grid, 128, 0, static_cast<cudaStream_t>(stream), 1, 1,
         static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ld_k, ld_v, k_cache, v_cache,
         k_scale, v_scale, segs, Hkv);
   else
-    kv_store_kernel<false><<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(nseg <= CHAIN_ROWS, kv_store_kernel<false>, grid, 128, 0, static_cast<cudaStream_t>(stream), 1, 1,
         static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), ld_k, ld_v, k_cache, v_cache,
         k_scale, v_scale, segs, Hkv);
   B2_LAUNCH_CHECK("kv_store");
@@ -618,21 +621,9 @@ B2_EXPORT int b2_paged_decode(const void* q, const void* k_cache, const void* v_
   if (nsplit == 1)
     while (cluster < DEC_MAX_CLUSTER && static_cast<long long>(B) * Hkv * cluster * 2 <= 2LL * num_sms() && cluster * 2 * (DEC_CHUNK / PAGE) <= max_blocks)
       cluster *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(B, Hkv, nsplit == 1 ? cluster : nsplit);
   // Two warps per CTA where there are many pairs anyway: CTAs of short contexts come and go faster.  256 sequences, 8 kv
   // heads, two / four warps, us: 128 tokens 31 / 39, 1024 tokens 130 / 125; 32 sequences of 2000 tokens 53 / 41.
   const int warps = static_cast<long long>(B) * Hkv >= 8LL * num_sms() ? 2 : 4;
-  cfg.blockDim = dim3(warps * 32, 1, 1);
-  cfg.dynamicSmemBytes = warps * (fp8 ? DecCfg<true>::RING : DecCfg<false>::RING);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = cluster;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
 #define B2_DECODE_LAUNCH_W(F8, GPV, WV)                                                                                   \
   do {                                                                                                              \
     auto kern = paged_decode_kernel<F8, GPV, WV>;                                                                   \
@@ -643,9 +634,11 @@ B2_EXPORT int b2_paged_decode(const void* q, const void* k_cache, const void* v_
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WV * DecCfg<F8>::RING);                \
       attr_set[dev & 63] = true;                                                                                    \
     }                                                                                                               \
-    cudaLaunchKernelEx(&cfg, kern, static_cast<const __nv_bfloat16*>(q), k_cache, v_cache, k_scale, v_scale,        \
-                       block_tables, context_lens, max_blocks, static_cast<__nv_bfloat16*>(out), part_o, part_ml,   \
-                       Hq, Hkv, partition, scale, nsplit == 1 ? 1 : 0);                                             \
+    /* not chained: waiting CTAs of this kernel hold shared memory that the products before it could use */ \
+    launch_chained(false, kern, dim3(B, Hkv, nsplit == 1 ? cluster : nsplit), WV * 32, WV * DecCfg<F8>::RING, stream, 1, \
+                   cluster, static_cast<const __nv_bfloat16*>(q), k_cache, v_cache, k_scale, v_scale, block_tables,  \
+                   context_lens, max_blocks, static_cast<__nv_bfloat16*>(out), part_o, part_ml, Hq, Hkv, partition, \
+                   scale, nsplit == 1 ? 1 : 0);                                                                     \
   } while (0)
 #define B2_DECODE_LAUNCH(F8, GPV)                     \
   do {                                                \

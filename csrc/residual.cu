@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(RES_THREADS) post_norm_kernel(float* __restric
                                                                 const float* __restrict__ ss, int parts, int nss,
                                                                 T* __restrict__ h, int ld, int n, float alpha, float eps) {
   __shared__ float scratch[32];
+  chain_wait();
+  chain_release();
   const size_t base = static_cast<size_t>(blockIdx.x) * ld;
   float f = 1.f;
   if (ss) {
@@ -583,7 +585,7 @@ B2_EXPORT int b2_post_norm(float* x, const float* y, const void* w, const void* 
   }
   int threads = (ld / 8 + 31) / 32 * 32;
   if (threads > RES_THREADS) threads = RES_THREADS;
-  B2_DISPATCH_T(is_f32, post_norm_kernel<T><<<M, threads, 0, static_cast<cudaStream_t>(stream)>>>(
+  B2_DISPATCH_T(is_f32, launch_chained(M <= CHAIN_ROWS, post_norm_kernel<T>, dim3(M), threads, 0, static_cast<cudaStream_t>(stream), 1, 1,
       x, y, static_cast<const T*>(w), static_cast<const T*>(b), ss, parts, nss, static_cast<T*>(h), ld, n, alpha, eps););
   B2_CHECK_LAUNCH("post_norm");
   return 0;
