@@ -483,7 +483,8 @@ class InferenceEngine:
             at += len(toks)
         tokens = [t for _, toks in entries for t in toks]
         ids = [i for i, _ in entries]
-        pick = torch.tensor(rows, dtype=torch.long, device=self.device)
+        # through pinned memory: a copy from pageable memory would wait for the step before, and the GPU then for the host
+        pick = self._stage("rows", torch.tensor(rows, dtype=torch.long))
         self.stats["steps"] += 1
         if all(c == 1 for c in counts):          # decode step
             logits = self.runner.forward(self._stage("feed", torch.tensor(tokens, dtype=torch.long)),
