@@ -106,6 +106,17 @@ def test_cluster_products(b_mn, M, N, K, bn, cluster):
     nv.assert_ok()
 
 
+@pytest.mark.parametrize("bn", [0, 128, 256])      # 0: the dispatch's own choice (a cluster)
+@pytest.mark.parametrize("M,N", [(5, 1028), (130, 36), (3, 20)])
+def test_residual_beside_fp32_rows_of_four(bn, M, N):
+    """Rows of 4 n elements: every other row of the bf16 addend starts 8 bytes off a vector of 16."""
+    from b200fw.ops import gemm
+    g = torch.Generator(device=DEV).manual_seed(8)
+    a, b, r = (torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for s in ((M, 2048), (N, 2048), (M, N)))
+    got, _ = _error(gemm(a, b, residual=r, out_dtype=torch.float32, bn=bn), a.double() @ b.double().t() + r.double())
+    assert got <= 1e-5, got      # 32-bit sums, as in test_cluster_products
+
+
 @pytest.mark.parametrize("act", ["silu", "relu2"])
 @pytest.mark.parametrize("M", [1, 33, 256])
 def test_products_with_few_rows_take_every_epilogue(act, M):
