@@ -155,6 +155,10 @@ __device__ __forceinline__ int snake_next(int w) {
 // nothing that it may read is written, before it.  chain_release lets the next chained kernel start; it is given once this
 // CTA is short of finishing, so that the next kernel's CTAs do not sit on registers that other streams could use.  Both do nothing
 // in a kernel that was launched, or is followed, in the ordinary way.
+// Parameters of a kernel that calls chain_wait which are read (in-place ones too) carry no __restrict__: on a const pointer it
+// promises that nobody writes the data as long as the kernel lives, on any pointer that the wait's memory clobber does not
+// concern it, and either lets the compiler load before the wait what the kernel before is still writing.
+// Pure outputs may carry it: what is stored depends on what was loaded.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -57,7 +57,7 @@ constexpr int RMS_THREADS = 256;
 constexpr int RMS_MAX_VEC = 4;  // up to 256*8*4 = 8192 columns kept in registers
 
 __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_fwd_kernel(
-    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+    const __nv_bfloat16* x, const __nv_bfloat16* w,
     __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float scratch[32];
   chain_wait();
@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_fwd_kernel(
   const __nv_bfloat16* xr = x + row * H;
   __nv_bfloat16* yr = y + row * H;
   float v[RMS_MAX_VEC][8];
+  uint4 wr[RMS_MAX_VEC];   // the weight is requested with the row: after the sum its latency would come on top
   float ss = 0.f;
   const int nvec = H / 8;
 #pragma unroll
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_fwd_kernel(
     const int c = threadIdx.x + i * RMS_THREADS;
     if (c < nvec) {
       load8(xr + c * 8, v[i]);
+      wr[i] = *reinterpret_cast<const uint4*>(w + c * 8);
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
     }
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_fwd_kernel(
     const int c = threadIdx.x + i * RMS_THREADS;
     if (c < nvec) {
       float wv[8], o[8];
-      load8(w + c * 8, wv);
+      raw8(wr[i], wv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = v[i][j] * rstd * wv[j];
       store8(yr + c * 8, o);
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_bwd_kernel(
 // ---------------------------------------------------------------------------------------------
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(
-    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+    const __nv_bfloat16* x, const __nv_bfloat16* w,
     __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int M, int H, float eps) {
   chain_wait();
   chain_release();
@@ -194,12 +196,14 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(
   for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < M; row += warps_per_grid) {
     const __nv_bfloat16* xr = x + static_cast<size_t>(row) * H;
     float v[NV][8];
+    uint4 wr[NV];   // requested with the row, as above
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int c = lane + i * 32;
       if (c < nvec) {
         load8(xr + c * 8, v[i]);
+        wr[i] = *reinterpret_cast<const uint4*>(w + c * 8);
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
       }
@@ -213,7 +217,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_warp_kernel(
       const int c = lane + i * 32;
       if (c < nvec) {
         float o[8], wv[8];
-        load8(w + c * 8, wv);
+        raw8(wr[i], wv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = v[i][j] * rstd * wv[j];
         store8(yr + c * 8, o);
@@ -392,12 +396,12 @@ __device__ __forceinline__ float sum16(float v) {   // over the 16 lanes that sh
 // output) are written there by the same warp, so the runner needs no separate store launch and K / V are not re-read.
 template <bool STORE>
 __global__ void __launch_bounds__(256) qknorm_rope_fwd_kernel(
-    const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ qw,
-    const __nv_bfloat16* __restrict__ kw, const int* __restrict__ pos,
-    const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+    const __nv_bfloat16* qkv, const __nv_bfloat16* qw,
+    const __nv_bfloat16* kw, const int* pos,
+    const float* cos_t, const float* sin_t,
     __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_out,
     float* __restrict__ rstd_out, int M, int Hq, int Hkv, int ld_qkv, float eps,
-    const int* __restrict__ slots, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache) {
+    const int* slots, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache) {
   chain_wait();
   chain_release();
   const int heads = Hq + Hkv;
@@ -566,7 +570,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_bwd_kernel(
 // ---------------------------------------------------------------------------------------------
 // SwiGLU on the fused gate|up projection output gu [M, 2I]: out = silu(gate) * up.
 // ---------------------------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ out,
                                   long long M, int I) {
   chain_wait();
   chain_release();

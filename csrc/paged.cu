@@ -34,9 +34,9 @@ __device__ __forceinline__ uint8_t float_to_fp8(float v) {
 // ---------------------------------------------------------------------------------------------
 template <bool FP8>
 __global__ void __launch_bounds__(128) kv_store_kernel(
-    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, int ld_k, int ld_v,
-    void* __restrict__ k_cache, void* __restrict__ v_cache, float* __restrict__ k_scale,
-    float* __restrict__ v_scale, const int* __restrict__ segs, int Hkv) {
+    const __nv_bfloat16* k, const __nv_bfloat16* v, int ld_k, int ld_v,
+    void* k_cache, void* v_cache, float* k_scale,
+    float* v_scale, const int* segs, int Hkv) {
   __shared__ float red[4];
   chain_wait();
   chain_release();
@@ -51,8 +51,13 @@ __global__ void __launch_bounds__(128) kv_store_kernel(
   const size_t tok_stride = static_cast<size_t>(Hkv) * HD;
   if (!FP8) {
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(which ? v_cache : k_cache);
-    for (int t = 0; t < count; ++t)
-      dst[base + (off + t) * tok_stride] = src[static_cast<size_t>(tok0 + t) * ld + h * HD + d];
+    __nv_bfloat16 rows[PAGE];   // all loads before the first store: the compiler may not move one over the other
+#pragma unroll
+    for (int t = 0; t < PAGE; ++t)
+      if (t < count) rows[t] = src[static_cast<size_t>(tok0 + t) * ld + h * HD + d];
+#pragma unroll
+    for (int t = 0; t < PAGE; ++t)
+      if (t < count) dst[base + (off + t) * tok_stride] = rows[t];
     return;
   }
   uint8_t* dst = reinterpret_cast<uint8_t*>(which ? v_cache : k_cache);

@@ -80,9 +80,9 @@ __global__ void __launch_bounds__(RES_THREADS) rmsnorm_f32_kernel(const float* _
 // x <- rms(alpha x + f y + b) w, and the same rounded to T in h (optional).  y: fp32 [M, ld]; b (optional): T [ld]; f is 1, or
 // the root of a norm over the reader's input that was left to this kernel: 1 / sqrt(sum_j ss[row, j] / nss + eps).
 template <typename T>
-__global__ void __launch_bounds__(RES_THREADS) post_norm_kernel(float* __restrict__ x, const float* __restrict__ y,
-                                                                const T* __restrict__ w, const T* __restrict__ b,
-                                                                const float* __restrict__ ss, int parts, int nss,
+__global__ void __launch_bounds__(RES_THREADS) post_norm_kernel(float* x, const float* y,
+                                                                const T* w, const T* b,
+                                                                const float* ss, int parts, int nss,
                                                                 T* __restrict__ h, int ld, int n, float alpha, float eps) {
   __shared__ float scratch[32];
   chain_wait();
