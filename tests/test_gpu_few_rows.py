@@ -117,6 +117,20 @@ def test_residual_beside_fp32_rows_of_four(bn, M, N):
     assert got <= 1e-5, got      # 32-bit sums, as in test_cluster_products
 
 
+@pytest.mark.parametrize("bn", [0, 128, 256])      # 0: the dispatch's own choice (a cluster for the smaller two)
+@pytest.mark.parametrize("M,N,K", [(5, 1024, 2048), (130, 72, 2048), (300, 776, 520), (3000, 1000, 256)])
+def test_addend_and_accumulation_together(bn, M, N, K):
+    """out += a b^T + residual, in both output types and by both kernels."""
+    from b200fw.ops import gemm
+    g = torch.Generator(device=DEV).manual_seed(9)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    a, b, r = rnd(M, K).to(torch.bfloat16), rnd(N, K).to(torch.bfloat16), rnd(M, N).to(torch.bfloat16)
+    for old in (rnd(M, N).mul(20).to(torch.bfloat16), rnd(M, N).mul(20)):
+        want = a.double() @ b.double().t() + old.double() + r.double()
+        got, floor = _error(gemm(a, b, out=old, accumulate=True, residual=r, bn=bn), want)
+        assert got <= (1.02 * floor if old.dtype == torch.bfloat16 else 0.0) + 1e-5, (got, floor)      # as in test_cluster_products
+
+
 @pytest.mark.parametrize("act", ["silu", "relu2"])
 @pytest.mark.parametrize("M", [1, 33, 256])
 def test_products_with_few_rows_take_every_epilogue(act, M):
