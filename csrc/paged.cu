@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
       }
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-      const int e = min(max(static_cast<int>(__float_as_uint(amax) >> 23), 127 - 100), 127 + 100);   // biased exponent
+      const int e = min(max(static_cast<int>(__float_as_uint(amax) >> 23), 127 - 100), 254);   // biased exponent
       const float to = __uint_as_float(static_cast<uint32_t>(127 + 13 + 127 - e) << 23);             // 2^(13 - (e - 127))
       qscale *= __uint_as_float(static_cast<uint32_t>(e - 13) << 23);                               // its reciprocal
 #pragma unroll
@@ -327,7 +327,9 @@ __global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
 #pragma unroll
   for (int j = 0; j < 16; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   float m = -INFINITY, l = 0.f, my_ks = 1.f, my_vs = 1.f;
-  int ev = 1;   // fp8: largest biased exponent of the value scales so far (acc is scaled by its inverse)
+  // fp8: largest biased exponent of the value scales so far (acc is scaled by its inverse).  It starts where 2^14 times the
+  // inverse is still finite and the last factor, 2^(ev - 127) / 2^14, still normal: a page may have the scale 0.
+  int ev = 16;
 
   for (int i = 0; warp + WARPS * i < tiles; ++i) {
     issue(i + Cfg::STAGES - 1);

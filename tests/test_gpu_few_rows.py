@@ -66,6 +66,33 @@ def test_decode_attention_over_clusters(fp8, Hq, Hkv, lens):
         assert got <= 1.02 * floor + 2e-5, (part, nsplit, got, floor)
 
 
+@pytest.mark.parametrize("v_exp", [[None, None], [None, 0], [0, None], [-90, -90], [-60, -90], [100, -20], [118, 118]])
+@pytest.mark.parametrize("q_exp", [-110, 0, 110])
+def test_fp8_decode_over_the_range_of_scales(v_exp, q_exp):
+    """Value scales of zero (None: an all-zero page as other writers leave it), tiny and large powers of two; queries whose scores
+    are nearly all zero, ordinary, or so large that one key takes everything."""
+    from b200fw.ops import paged_decode_attention
+    g = torch.Generator(device=DEV).manual_seed(10)
+    Hkv, n = 2, 300
+    pages = -(-n // 16)
+    kc, vc = (torch.randn(pages, 16, Hkv, 128, device=DEV, generator=g).to(torch.float8_e4m3fn).view(torch.uint8) for _ in range(2))
+    ks = torch.full((pages, Hkv), 2.0 ** -8, device=DEV)
+    vs = torch.zeros(pages, Hkv, device=DEV)
+    for i, e in enumerate(v_exp):      # pages take turns
+        vs[i::2] = 0.0 if e is None else 2.0 ** e
+    q = (torch.randn(1, 4 * 128, device=DEV, generator=g) * 2.0 ** q_exp).to(torch.bfloat16)
+    bt, cl = torch.arange(pages, device=DEV).int().view(1, -1), torch.tensor([n], device=DEV).int()
+    want = _decode_reference(q, kc, vc, bt, [n], 4, ks, vs)
+    for part, nsplit in ((0, 1), (64, 5)):
+        out = paged_decode_attention(q, kc, vc, bt, cl, 4, k_scale=ks, v_scale=vs, partition=part, nsplit=nsplit)
+        assert bool(torch.isfinite(out).all())
+        if v_exp == [None, None]:
+            assert not out.any()
+            continue
+        got, floor = _error(out, want)
+        assert got <= 1.02 * floor + 2e-5, (part, got, floor)      # as in test_decode_attention_over_clusters
+
+
 def test_decode_attention_of_many_pairs_and_unaligned_queries():
     """So many (sequence, kv head) pairs that CTAs of two warps run; queries two bytes off a vector's alignment."""
     from b200fw.ops import paged_decode_attention
