@@ -128,7 +128,8 @@ __global__ void kv_gather_kernel(const void* __restrict__ k_cache, const void* _
 //   scores:  A = the query heads, one per row (rows r and r + GP hold the same head), B = the page's keys.
 //   output:  A = the probabilities, B = the page's values.  Probabilities keep 24 bits: p = hi + mid + lo in the 16-bit type,
 //            and rows r, r + GP, r + 2 GP of A are those three parts of the same head, so the split costs no product of its
-//            own up to four heads (GP = 8: a second one).  The rows of a head are added up once, at the end.
+//            own up to four heads (GP = 8: a second one).  The rows of a head are added up once, at the end; where the first
+//            is infinite (16-bit values may be), it alone counts.
 // Contraction indices may be permuted freely, so both operands are read from shared memory 16 bytes per lane: lane
 // (r = lane / 4, c = lane % 4) owns the dims of chunks c, c + 4, .. of key r, and dims 16 r .. 16 r + 15 of the values of
 // tokens 2 c, 2 c + 1, 2 c + 8, 2 c + 9.  The chunk swizzle below makes both patterns free of bank conflicts.
@@ -166,32 +167,47 @@ __device__ __forceinline__ void dec_mma(float (&d)[4], uint32_t a0, uint32_t a1,
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// two floats in the operand type (first one in the low half), and back
-template <bool FP8>
+// two floats as halves (first one in the low half), and back
 __device__ __forceinline__ uint32_t dec_pack(float x, float y) {
-  if (!FP8) return pack_bf16x2(x, y);
   const __half2 h = __floats2half2_rn(x, y);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
-template <bool FP8>
-__device__ __forceinline__ float2 dec_unpack(uint32_t u) {
-  if (!FP8) return unpack_bf16x2(u);
-  return __half22float2(*reinterpret_cast<const __half2*>(&u));
-}
-// Part `part` of the pair (x, y): 0 the rounded value, 1 what rounding left, 2 what is left after both; none beyond.
+__device__ __forceinline__ float2 dec_unpack(uint32_t u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
+// Part `part` of the pair (x, y): 0 the leading bits, 1 the leading ones of the rest, 2 what is left after both; none beyond.
+// fp16 parts are rounded.  bf16 parts are cut off, 8 bits each: of a probability none is negative, and three are all of it.
 template <bool FP8>
 __device__ __forceinline__ uint32_t dec_part(float x, float y, int part) {
-  uint32_t u = dec_pack<FP8>(x, y);
+  if (!FP8) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (part > i) {
+        x -= __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+        y -= __uint_as_float(__float_as_uint(y) & 0xFFFF0000u);
+      }
+    }
+    return part > 2 ? 0u : __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632u);
+  }
+  uint32_t u = dec_pack(x, y);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     if (part > i) {
-      const float2 f = dec_unpack<FP8>(u);
+      const float2 f = dec_unpack(u);
       x -= f.x;
       y -= f.y;
-      u = dec_pack<FP8>(x, y);
+      u = dec_pack(x, y);
     }
   }
   return part > 2 ? 0u : u;
+}
+// The last part where it has no rows of its own and is added to the first one's (eight heads).  A bf16 value may be infinite: the
+// part is then not 0 unless the probability is, so that both rows' products are the same infinity.
+template <bool FP8>
+__device__ __forceinline__ uint32_t dec_last_part(float x, float y) {
+  if (FP8) return dec_part<FP8>(x, y, 2);
+  const uint32_t u = dec_part<FP8>(x, y, 2);
+  const float2 f = unpack_bf16x2(u);
+  const float tiny = 7.888609e-31f;   // 2^-100
+  return __byte_perm(__float_as_uint(fmaxf(f.x, fminf(x, tiny))), __float_as_uint(fmaxf(f.y, fminf(y, tiny))), 0x7632u);
 }
 // two e4m3 bytes (the low half of w) as two halves
 __device__ __forceinline__ uint32_t dec_fp8x2(uint32_t w) {
@@ -318,7 +334,7 @@ __global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float2 f = unpack_bf16x2(qa[i]);
-        qa[i] = dec_pack<true>(f.x * to, f.y * to);
+        qa[i] = dec_pack(f.x * to, f.y * to);
       }
     }
   }
@@ -413,7 +429,7 @@ __global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
     }
     const uint32_t a0 = dec_part<FP8>(s[0], s[1], part_a), a2 = dec_part<FP8>(s[2], s[3], part_a);
     const uint32_t a1 = GP >= 4 ? dec_part<FP8>(s[0], s[1], part_b) : 0u, a3 = GP >= 4 ? dec_part<FP8>(s[2], s[3], part_b) : 0u;
-    const uint32_t x0 = GP == 8 ? dec_part<FP8>(s[0], s[1], 2) : 0u, x2 = GP == 8 ? dec_part<FP8>(s[2], s[3], 2) : 0u;
+    const uint32_t x0 = GP == 8 ? dec_last_part<FP8>(s[0], s[1]) : 0u, x2 = GP == 8 ? dec_last_part<FP8>(s[2], s[3]) : 0u;
     // ---- output dims 16 n + j of n-tile j
 #pragma unroll
     for (int h = 0; h < Cfg::CPR / 8; ++h) {
@@ -465,7 +481,9 @@ __global__ void __launch_bounds__(WARPS * 32) paged_decode_kernel(
       o0 += __shfl_xor_sync(0xffffffffu, o0, d);
       o1 += __shfl_xor_sync(0xffffffffu, o1, d);
     }
-    if (r < GP) {
+    if (r < GP) {   // this lane's row r is the high part of head r: where it is infinite, the other parts are 0 * inf or -inf
+      o0 = fabsf(acc[j][0]) < INFINITY ? o0 : acc[j][0];
+      o1 = fabsf(acc[j][1]) < INFINITY ? o1 : acc[j][1];
       *reinterpret_cast<float2*>(wo + r * PITCH + 8 * j + 2 * c) = make_float2(o0 * unit, o1 * unit);
     }
   }

@@ -93,6 +93,28 @@ def test_fp8_decode_over_the_range_of_scales(v_exp, q_exp):
         assert got <= 1.02 * floor + 2e-5, (part, got, floor)      # as in test_decode_attention_over_clusters
 
 
+@pytest.mark.parametrize("G", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("n,split", [(5, (0, 1)), (200, (0, 1)), (200, (64, 4))])
+def test_decode_attention_with_infinite_values(G, n, split):
+    """An infinity (or NaN) in one channel of one cached value reaches that channel of the output and nothing else."""
+    from b200fw.ops import paged_decode_attention
+    g = torch.Generator(device=DEV).manual_seed(11)
+    pages, Hkv = -(-n // 16), 2
+    kc, vc = (torch.randn(pages, 16, Hkv, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    flat = vc.view(-1, Hkv, 128)
+    flat[1, 0, 3] = flat[n - 1, 0, 100] = math.inf
+    flat[2, 0, 64] = flat[3, 1, 5] = -math.inf
+    flat[4, 1, 127] = math.nan
+    q = torch.randn(1, G * Hkv * 128, device=DEV, generator=g).mul(0.5).to(torch.bfloat16)
+    bt, cl = torch.arange(pages, device=DEV).int().view(1, -1), torch.tensor([n], device=DEV).int()
+    want = _decode_reference(q, kc, vc, bt, [n], G * Hkv, None, None)
+    out = paged_decode_attention(q, kc, vc, bt, cl, G * Hkv, partition=split[0], nsplit=split[1]).double()
+    odd = ~torch.isfinite(want)
+    assert int(odd.sum()) == 5 * G and torch.equal(out[odd].nan_to_num(7.0), want[odd].nan_to_num(7.0))
+    got, floor = _error(out[~odd], want[~odd])
+    assert got <= 1.02 * floor + 2e-5, (got, floor)      # as in test_decode_attention_over_clusters
+
+
 def test_decode_attention_of_many_pairs_and_unaligned_queries():
     """So many (sequence, kv head) pairs that CTAs of two warps run; queries two bytes off a vector's alignment."""
     from b200fw.ops import paged_decode_attention
