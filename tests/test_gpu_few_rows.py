@@ -237,3 +237,24 @@ def test_attention_backward_of_ragged_rows():
     for a, b in ((q, qd), (k, kd), (v, vd)):
         # P and dS are bf16 operands of the gradient products: 2^-9 each, a few of them added up
         assert _error(a.grad, b.grad)[0] < 1e-2
+
+
+@pytest.mark.parametrize("bn", [0, 128])      # cluster, persistent kernel
+def test_failed_launch_is_reported_once(bn):
+    """A product on a stream whose capture has been invalidated is refused by the runtime; the next operation is not."""
+    import ctypes
+    from b200fw.ops import gemm, rmsnorm
+    a, b, w = (torch.ones(*s, device=DEV, dtype=torch.bfloat16) for s in ((5, 2048), (1024, 2048), (1024,)))
+    out, want = gemm(a, b, bn=bn), rmsnorm(torch.ones(5, 1024, device=DEV, dtype=torch.bfloat16), w)
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL("libcudart.so.12")
+    stream = torch.cuda.Stream()
+    raw, graph = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+    with torch.cuda.stream(stream):
+        assert rt.cudaStreamBeginCapture(raw, 2) == 0
+        assert rt.cudaStreamSynchronize(raw) != 0      # not allowed while capturing: the capture is invalid from here on
+        with pytest.raises(RuntimeError, match="launch failed"):
+            gemm(a, b, out=out, bn=bn)
+        assert rt.cudaStreamEndCapture(raw, ctypes.byref(graph)) != 0
+    rt.cudaGetLastError()
+    assert torch.equal(rmsnorm(out.mul(0).add(1), w), want)
