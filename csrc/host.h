@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstdlib>
+
 #define B2_EXPORT extern "C" __attribute__((visibility("default")))
 
 namespace b2 {
@@ -41,6 +43,16 @@ inline int num_sms() {
   cudaGetDevice(&dev);
   if (n[dev] == 0) cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev);
   return n[dev];
+}
+
+// B200FW_BATCH_INVARIANT=1: a row's sums are taken in one order, however many rows or sequences there are beside it: no products
+// or contexts dealt to a cluster, which the dispatch does by how many there are.
+inline bool batch_invariant() {
+  static const bool on = [] {
+    const char* e = std::getenv("B200FW_BATCH_INVARIANT");
+    return e != nullptr && e[0] == '1';
+  }();
+  return on;
 }
 
 // Steps of few rows (decoding, single short examples) are chains of short kernels: the launch, barrier set-up and first copies

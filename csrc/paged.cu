@@ -643,12 +643,12 @@ B2_EXPORT int b2_paged_decode(const void* q, const void* k_cache, const void* v_
   // head) pairs of 1024 tokens 12.9 / 9.6 / 7.6 / 6.3; 64 pairs of up to 8192 80.3 / 45.5 / 41.8 / 45.5; 256 pairs of up to 2000
   // 41.3 / 48.2 / 58.5 / 87.4.
   int cluster = 1;
-  if (nsplit == 1)
+  if (nsplit == 1 && !batch_invariant())
     while (cluster < DEC_MAX_CLUSTER && static_cast<long long>(B) * Hkv * cluster * 2 <= 2LL * num_sms() && cluster * 2 * (DEC_CHUNK / PAGE) <= max_blocks)
       cluster *= 2;
   // Two warps per CTA where there are many pairs anyway: CTAs of short contexts come and go faster.  256 sequences, 8 kv
   // heads, two / four warps, us: 128 tokens 31 / 39, 1024 tokens 130 / 125; 32 sequences of 2000 tokens 53 / 41.
-  const int warps = static_cast<long long>(B) * Hkv >= 8LL * num_sms() ? 2 : 4;
+  const int warps = static_cast<long long>(B) * Hkv >= 8LL * num_sms() && !batch_invariant() ? 2 : 4;
 #define B2_DECODE_LAUNCH_W(F8, GPV, WV)                                                                                   \
   do {                                                                                                              \
     auto kern = paged_decode_kernel<F8, GPV, WV>;                                                                   \

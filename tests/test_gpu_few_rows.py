@@ -258,3 +258,40 @@ def test_failed_launch_is_reported_once(bn):
         assert rt.cudaStreamEndCapture(raw, ctypes.byref(graph)) != 0
     rt.cudaGetLastError()
     assert torch.equal(rmsnorm(out.mul(0).add(1), w), want)
+
+
+_SAME_IN_ANY_BATCH = """
+import torch
+from b200fw import ops
+g = torch.Generator(device="cuda").manual_seed(12)
+rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+for n, k in ((1024, 3072), (4096, 1024), (2560, 9728)):
+    x, w, r = rnd(1100, k), rnd(n, k), rnd(1100, n)
+    alone = ops.linear(x[:1], w, r[:1])
+    for m in (2, 64, 130, 1100):
+        assert torch.equal(ops.linear(x[:m], w, r[:m])[:1], alone), (n, k, m)
+B, Hq, Hkv, n = 300, 16, 8, 700
+pages = -(-n // 16)
+kc, vc, q = rnd(4 * pages, 16, Hkv, 128), rnd(4 * pages, 16, Hkv, 128), rnd(B, Hq * 128)
+table = (torch.arange(pages)[None] + pages * (torch.arange(B) % 4)[:, None]).int().cuda()
+lens = torch.full((B,), n, dtype=torch.int32, device="cuda")
+for fp8 in (False, True):
+    if fp8:
+        kc, vc = (t.to(torch.float8_e4m3fn).view(torch.uint8) for t in (kc, vc))
+    s = torch.rand(4 * pages, Hkv, device="cuda", generator=g) if fp8 else None
+    run = lambda b: ops.paged_decode_attention(q[:b], kc, vc, table[:b].contiguous(), lens[:b], Hq, k_scale=s, v_scale=s)
+    alone = run(1)
+    for b in (3, 20, 70, B):
+        assert torch.equal(run(b)[:1], alone), (fp8, b)
+"""
+
+
+def test_results_do_not_depend_on_the_batch_where_asked():
+    """With B200FW_BATCH_INVARIANT=1 (read once, hence a process of its own) a row is the same alone and among others."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SAME_IN_ANY_BATCH], cwd=root, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "B200FW_BATCH_INVARIANT": "1"})
+    assert r.returncode == 0, r.stderr[-2000:]
