@@ -53,6 +53,7 @@ class ModelRunner:
         self.dtype = next(model.parameters()).dtype
         self.partition_size, self.enable_partitioned = partition_size, enable_partitioned
         self.block_size = pool.block_size
+        self.num_sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 0
         self.forward_calls = 0
         self.fuse_kv_store = True     # norm + RoPE + cache store in one launch for 16-bit caches (False: two launches)
 
@@ -168,30 +169,25 @@ class ModelRunner:
 
         return InferenceContext(
             is_prefill=False, num_seqs=B, block_tables=dev(bt), context_lens=dev(ctx_lens),
-            max_context_len=int(lens.max()) if n else 0, store_segments=dev(segs), positions=dev(pos),
-            slot_mapping=dev(slots))
+            max_context_len=int(lens.max()) if n else 0, total_k=int(lens.sum()), store_segments=dev(segs),
+            positions=dev(pos), slot_mapping=dev(slots))
 
     # ---- forward -----------------------------------------------------------------------------------------
     def _split_plan(self, ctx: InferenceContext) -> Tuple[int, int]:
         if self.enable_partitioned and ctx.max_context_len > self.partition_size:
             part = max(64, self.partition_size // 64 * 64)
             return part, (ctx.max_context_len + part - 1) // part
-        if getattr(self, "balance_splits", False) and ctx.max_context_len > 256:
-            # One CTA per (sequence, kv head group) leaves the last of ~3.5 waves (256 sequences x 8 kv heads over
-            # 148 SMs x 4 resident CTAs) mostly empty, and a long sequence pins its CTA while the others finish.
-            # Splitting every sequence into a few partitions gives ~8 waves of shorter CTAs; the exact log-sum-exp
-            # merge costs one small kernel.
-            cfg = self.cfg
-            g = cfg.num_heads // cfg.num_kv_heads
-            gh = 4 if g % 4 == 0 and not self.pool.fp8 else (2 if g % 2 == 0 else 1)
-            ctas = ctx.num_seqs * cfg.num_kv_heads * (g // gh)
-            want = 8 * 148 * 4
-            if ctas < want:
-                nsplit = min((ctx.max_context_len + 255) // 256, -(-want // ctas))
-                if nsplit > 1:
-                    part = -(-ctx.max_context_len // nsplit)
-                    part = (part + 63) // 64 * 64
-                    return part, (ctx.max_context_len + part - 1) // part
+        if getattr(self, "balance_splits", False):
+            # Up to one (sequence, kv head) pair per SM the kernel deals a context to a cluster by itself, and contexts of
+            # like lengths keep every SM busy.  Left are long contexts among shorter ones, which pin their CTAs while the
+            # others have finished: four parts and the exact log-sum-exp merge.  us, unsplit / four parts, 8 kv heads, bf16 and
+            # fp8 cache: 64 sequences of 100 to 4000 tokens 124 / 112, 112 / 93; 24 of 100 to 30000 428 / 286, 528 / 239; 256 of
+            # 100 to 4000 386 / 378, 366 / 352; but 128 of 3000 to 4000 297 / 302, 236 / 253; 256 of 512 to 1024 148 / 159,
+            # 127 / 144 (three parts).
+            pairs, longest = ctx.num_seqs * self.cfg.num_kv_heads, ctx.max_context_len
+            if pairs > self.num_sms and longest > 2048 and 2 * longest * ctx.num_seqs > 3 * ctx.total_k:
+                part = (-(-longest // 4) + 63) // 64 * 64
+                return part, -(-longest // part)
         return 0, 1
 
     @torch.no_grad()

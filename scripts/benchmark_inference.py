@@ -45,7 +45,7 @@ def parse_args(argv=None):
     ap.add_argument("--profile-decode-steps", type=int, default=0,
                     help="bracket this many decode steps with cudaProfilerStart/Stop (for `ncu --profile-from-start off`)")
     ap.add_argument("--balance-splits", action="store_true",
-                    help="split every sequence's keys over a few CTAs when the decode grid would fill only a few waves")
+                    help="split every sequence's keys over a few CTAs when contexts of very unequal lengths are decoded together")
     ap.add_argument("--no-async-decode", dest="async_decode", action="store_false",
                     help="read every step's sampled ids back before the next step is launched")
     return ap.parse_args(argv)

@@ -33,6 +33,37 @@ def oracle(model):
     return InferenceEngine(cfg, model).initialize().generate(PROMPTS, max_tokens=10)
 
 
+@pytest.mark.parametrize("lens,kv_heads,plan", [
+    ([1000, 1500, 2000] * 10, 8, (0, 1)),             # the kernel's own time is best: lengths alike, none of them long
+    ([3000, 4000] * 64, 8, (0, 1)),
+    ([4000] + [100] * 17, 8, (0, 1)),                 # 144 pairs on 148 SMs: a cluster per context
+    ([4000] + [100] * 18, 8, (1024, 4)),              # a long context among short ones
+    ([2049] + [1] * 40, 4, (576, 4)),
+    ([2048] + [1] * 40, 4, (0, 1)),
+    ([30000] + [500] * 40, 2, (0, 1)),
+])
+def test_balanced_splits_are_for_unequal_contexts(lens, kv_heads, plan):
+    """``decode_balance_splits`` against the grid of the decode kernel: one CTA per (sequence, kv head), or a cluster of them."""
+    from types import SimpleNamespace as NS
+
+    from b200fw.infer.runner import ModelRunner
+    r = NS(enable_partitioned=False, balance_splits=True, num_sms=148, cfg=NS(num_heads=8 * kv_heads, num_kv_heads=kv_heads))
+    ctx = NS(num_seqs=len(lens), max_context_len=max(lens), total_k=sum(lens))
+    assert ModelRunner._split_plan(r, ctx) == plan
+    r.balance_splits = False
+    assert ModelRunner._split_plan(r, ctx) == (0, 1)
+
+
+def test_balanced_splits_decode_the_same_tokens(model, oracle):
+    e = _engine(model, decode_balance_splits=True)
+    e.runner.num_sms = 1
+    r = e.runner
+    seen, plan = [], r._split_plan
+    r._split_plan = lambda ctx: seen.append((ctx.num_seqs, ctx.max_context_len, ctx.total_k)) or plan(ctx)
+    assert e.generate(PROMPTS, max_tokens=10) == oracle
+    assert seen and all(longest <= total <= n * longest for n, longest, total in seen)
+
+
 def test_kv_manager_allocation_rollback_and_double_free():
     pool = BlockPool(8, 16, 1, 1, 8, torch.float32, "cpu")
     mgr = KVCacheManager(pool, 16)
