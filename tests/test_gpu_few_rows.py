@@ -115,6 +115,35 @@ def test_decode_attention_with_infinite_values(G, n, split):
     assert got <= 1.02 * floor + 2e-5, (got, floor)      # as in test_decode_attention_over_clusters
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,lens", [
+    (16, 8, [4999, 1, 2100, 2049, 4096, 15, 3000, 700]),              # 64 pairs: clusters of four
+    (32, 8, [2561, 2560, 5000] + [130] * 13),                         # 128 pairs: clusters of two, over 32 pages a warp
+    (8, 4, [2048, 2049, 2064, 2065, 4500, 4112] + [33] * 58),         # 256 pairs: four warps a context
+    (12, 4, [1024, 1025, 1040, 1041, 2300, 2072] + [40] * 294),       # 1200 pairs: two warps a context
+])
+def test_decode_attention_of_long_contexts(fp8, Hq, Hkv, lens):
+    """Every cluster size, and more than 32 pages a warp: page numbers and scales are then fetched again."""
+    from b200fw.ops import paged_decode_attention
+    g = torch.Generator(device=DEV).manual_seed(13)
+    need = [-(-n // 16) for n in lens]
+    blocks = sum(need)
+    kc, vc = (torch.randn(blocks, 16, Hkv, 128, device=DEV, generator=g) for _ in range(2))
+    kc, vc = (t.to(torch.float8_e4m3fn).view(torch.uint8) if fp8 else t.to(torch.bfloat16) for t in (kc, vc))
+    ks, vs = (10.0 ** (-2 + 2 * torch.rand(blocks, Hkv, device=DEV, generator=g)) if fp8 else None for _ in range(2))
+    perm = torch.randperm(blocks, device=DEV, generator=g).int()
+    bt = torch.full((len(lens), max(need)), -1, dtype=torch.int32, device=DEV)
+    at = 0
+    for b, n in enumerate(need):
+        bt[b, :n] = perm[at:at + n]
+        at += n
+    q = torch.randn(len(lens), Hq * 128, device=DEV, generator=g).to(torch.bfloat16)
+    cl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    got, floor = _error(paged_decode_attention(q, kc, vc, bt, cl, Hq, k_scale=ks, v_scale=vs),
+                        _decode_reference(q, kc, vc, bt, lens, Hq, ks, vs))
+    assert got <= 1.02 * floor + 2e-5, (got, floor)      # as in test_decode_attention_over_clusters
+
+
 def test_decode_attention_of_many_pairs_and_unaligned_queries():
     """So many (sequence, kv head) pairs that CTAs of two warps run; queries two bytes off a vector's alignment."""
     from b200fw.ops import paged_decode_attention
