@@ -798,14 +798,14 @@ B2_EXPORT int b2_attn_bwd(const void* q, const void* k, const void* v, const voi
   }
   const uint64_t T = static_cast<uint64_t>(B) * S;
   const uint64_t wq = static_cast<uint64_t>(Hq) * 128, wk = static_cast<uint64_t>(Hkv) * 128;
-  const CUtensorMap* tq128 = tensor_map_2d_bf16(q, T, wq, wq, 128, 64);
-  const CUtensorMap* tq64 = tensor_map_2d_bf16(q, T, wq, wq, 64, 64);
-  const CUtensorMap* tdo128 = tensor_map_2d_bf16(d_out, T, wq, wq, 128, 64);
-  const CUtensorMap* tdo64 = tensor_map_2d_bf16(d_out, T, wq, wq, 64, 64);
-  const CUtensorMap* tk128 = tensor_map_2d_bf16(k, T, wk, wk, 128, 64);
-  const CUtensorMap* tk64 = tensor_map_2d_bf16(k, T, wk, wk, 64, 64);
-  const CUtensorMap* tv128 = tensor_map_2d_bf16(v, T, wk, ld_v, 128, 64);
-  const CUtensorMap* tv64 = tensor_map_2d_bf16(v, T, wk, ld_v, 64, 64);
+  const TensorMap tq128 = tensor_map_2d_bf16(q, T, wq, wq, 128, 64);
+  const TensorMap tq64 = tensor_map_2d_bf16(q, T, wq, wq, 64, 64);
+  const TensorMap tdo128 = tensor_map_2d_bf16(d_out, T, wq, wq, 128, 64);
+  const TensorMap tdo64 = tensor_map_2d_bf16(d_out, T, wq, wq, 64, 64);
+  const TensorMap tk128 = tensor_map_2d_bf16(k, T, wk, wk, 128, 64);
+  const TensorMap tk64 = tensor_map_2d_bf16(k, T, wk, wk, 64, 64);
+  const TensorMap tv128 = tensor_map_2d_bf16(v, T, wk, ld_v, 128, 64);
+  const TensorMap tv64 = tensor_map_2d_bf16(v, T, wk, ld_v, 64, 64);
   if (!tq128 || !tq64 || !tdo128 || !tdo64 || !tk128 || !tk64 || !tv128 || !tv64) return 2;
   int* status = status_ptr();
   if (!status) return 3;

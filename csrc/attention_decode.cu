@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p,
 }
 
 template <int HALVES, int QP, int NG, bool EXACT, bool FEW>
-static int launch_form(DecodeParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int grid, cudaStream_t stream) {
+static int launch_form(DecodeParams& p, const TensorMap& tk, const TensorMap& tv, int grid, cudaStream_t stream) {
   constexpr int KT = 64 / HALVES;
   auto kern = decode_attn_kernel<HALVES, QP, NG, EXACT, FEW>;
   int stages = 8;
@@ -596,7 +596,7 @@ static int launch_form(DecodeParams& p, const CUtensorMap* tk, const CUtensorMap
   return 0;
 }
 template <int HALVES, int QP, int NG, bool EXACT>
-static int launch_decode(DecodeParams& p, const CUtensorMap* tk, const CUtensorMap* tv, int grid, cudaStream_t stream) {
+static int launch_decode(DecodeParams& p, const TensorMap& tk, const TensorMap& tv, int grid, cudaStream_t stream) {
   return p.heads * p.maps <= 8 ? launch_form<HALVES, QP, NG, EXACT, true>(p, tk, tv, grid, stream)
                                : launch_form<HALVES, QP, NG, EXACT, false>(p, tk, tv, grid, stream);
 }
@@ -655,7 +655,7 @@ B2_EXPORT int b2_decode_attention(const void* q, const void* kc, const void* vc,
     const uint32_t box[3] = {64, 1, AD_PAGE};
     return tensor_map_nd_bf16(base, 3, dims, strides, box, 3);
   };
-  const CUtensorMap *tk = map(kc, R), *tv = vc ? map(vc, C) : tk;
+  const TensorMap tk = map(kc, R), tv = vc ? map(vc, C) : tk;
   if (!tk || !tv) return 2;
   if (vc && R == 128 && C == 128) return launch_decode<1, 4, 1, true>(p, tk, tv, grid, st);
   if (vc) return R == 256 && C == 128 ? launch_decode<1, 8, 1, true>(p, tk, tv, grid, st) : launch_decode<1, 8, 1, false>(p, tk, tv, grid, st);

@@ -719,9 +719,9 @@ B2_EXPORT int b2_attn_fwd_varlen(const void* q, const void* k, const void* v, vo
     }
     configured[dev] = true;
   }
-  const CUtensorMap* tq = tensor_map_2d_bf16(q, total_q, static_cast<uint64_t>(Hq) * 128, static_cast<uint64_t>(Hq) * 128, 128, 64);
-  const CUtensorMap* tk = tensor_map_2d_bf16(k, total_k, static_cast<uint64_t>(Hkv) * 128, ld_k, 128, 64);
-  const CUtensorMap* tv = tensor_map_2d_bf16(v, total_k, static_cast<uint64_t>(Hkv) * 128, ld_v, 128, 64);
+  const TensorMap tq = tensor_map_2d_bf16(q, total_q, static_cast<uint64_t>(Hq) * 128, static_cast<uint64_t>(Hq) * 128, 128, 64);
+  const TensorMap tk = tensor_map_2d_bf16(k, total_k, static_cast<uint64_t>(Hkv) * 128, ld_k, 128, 64);
+  const TensorMap tv = tensor_map_2d_bf16(v, total_k, static_cast<uint64_t>(Hkv) * 128, ld_v, 128, 64);
   if (!tq || !tk || !tv) return 2;
   int* status = status_ptr();
   if (!status) return 3;
@@ -768,9 +768,9 @@ B2_EXPORT int b2_attn_fwd_paged(const void* q, const void* k_cache, const void* 
     configured[dev] = true;
   }
   const uint64_t W = static_cast<uint64_t>(Hkv) * 128;
-  const CUtensorMap* tq = tensor_map_2d_bf16(q, total_q, static_cast<uint64_t>(Hq) * 128, static_cast<uint64_t>(Hq) * 128, 128, 64);
-  const CUtensorMap* tk = tensor_map_2d_bf16(k_cache, static_cast<uint64_t>(num_blocks) * 16, W, W, 16, 64);
-  const CUtensorMap* tv = tensor_map_2d_bf16(v_cache, static_cast<uint64_t>(num_blocks) * 16, W, W, 16, 64);
+  const TensorMap tq = tensor_map_2d_bf16(q, total_q, static_cast<uint64_t>(Hq) * 128, static_cast<uint64_t>(Hq) * 128, 128, 64);
+  const TensorMap tk = tensor_map_2d_bf16(k_cache, static_cast<uint64_t>(num_blocks) * 16, W, W, 16, 64);
+  const TensorMap tv = tensor_map_2d_bf16(v_cache, static_cast<uint64_t>(num_blocks) * 16, W, W, 16, 64);
   if (!tq || !tk || !tv) return 2;
   int* status = status_ptr();
   if (!status) return 3;
@@ -816,10 +816,10 @@ B2_EXPORT int b2_attn_fwd_paged_ext(const void* q, const void* k_cache, const vo
     const uint32_t box[3] = {64, 1, box_rows};
     return tensor_map_nd_bf16(base, 3, dims, strides, box, 3);
   };
-  const CUtensorMap* tq = map3(q, total_q, static_cast<uint64_t>(Hq) * maps, dkp, ld_q, 128);
-  const CUtensorMap* tk = map3(k_cache, static_cast<uint64_t>(num_blocks) * 16, static_cast<uint64_t>(Hkv) * maps, dkp,
+  const TensorMap tq = map3(q, total_q, static_cast<uint64_t>(Hq) * maps, dkp, ld_q, 128);
+  const TensorMap tk = map3(k_cache, static_cast<uint64_t>(num_blocks) * 16, static_cast<uint64_t>(Hkv) * maps, dkp,
                                static_cast<uint64_t>(Hkv) * maps * dkp, 16);
-  const CUtensorMap* tv = map3(v_cache, static_cast<uint64_t>(num_blocks) * 16, Hkv, dvp, static_cast<uint64_t>(Hkv) * dvp, 16);
+  const TensorMap tv = map3(v_cache, static_cast<uint64_t>(num_blocks) * 16, Hkv, dvp, static_cast<uint64_t>(Hkv) * dvp, 16);
   if (!tq || !tk || !tv) return 2;
   int* status = status_ptr();
   if (!status) return 3;

@@ -86,13 +86,13 @@ struct MapKeyHash {
   }
 };
 
-// Entries are heap-allocated and never move, so returned pointers stay valid.
-static std::unordered_map<MapKey, CUtensorMap*, MapKeyHash> g_maps;
+static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
+constexpr size_t MAX_MAPS = 65536;
 
-const CUtensorMap* tensor_map_nd_bf16(const void* base, int rank, const uint64_t* dims,
-                                      const uint64_t* strides_bytes, const uint32_t* box,
-                                      int swizzle) {
+TensorMap tensor_map_nd_bf16(const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
+                             int swizzle) {
   ensure_thread_context();
+  TensorMap out;
   MapKey key;
   memset(&key, 0, sizeof(key));
   int dev = 0;
@@ -106,13 +106,14 @@ const CUtensorMap* tensor_map_nd_bf16(const void* base, int rank, const uint64_t
   }
   std::lock_guard<std::mutex> lock(g_mu);
   auto it = g_maps.find(key);
-  if (it != g_maps.end()) return it->second;
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return nullptr;
-  if (g_maps.size() > 65536) {  // unbounded growth guard: drop everything, maps are cheap to rebuild
-    for (auto& kv : g_maps) delete kv.second;
-    g_maps.clear();
+  if (it != g_maps.end()) {
+    out.map = it->second;
+    out.ok = true;
+    return out;
   }
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return out;
+  if (g_maps.size() >= MAX_MAPS) g_maps.clear();   // drop everything: maps are cheap to rebuild, and every caller has copies
   cuuint64_t gdim[4];
   cuuint64_t gstr[3];
   cuuint32_t bx[4];
@@ -126,23 +127,21 @@ const CUtensorMap* tensor_map_nd_bf16(const void* base, int rank, const uint64_t
                           : swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_64B
                           : swizzle == 1 ? CU_TENSOR_MAP_SWIZZLE_32B
                                          : CU_TENSOR_MAP_SWIZZLE_NONE;
-  CUtensorMap* m = new CUtensorMap;
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank),
+  CUresult r = fn(&out.map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank),
                   const_cast<void*>(base), gdim, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed: code %d (base %p rank %d dims %llu %llu box %u %u)",
               static_cast<int>(r), base, rank, (unsigned long long)dims[0],
               (unsigned long long)(rank > 1 ? dims[1] : 0), box[0], rank > 1 ? box[1] : 0);
-    delete m;
-    return nullptr;
+    return out;
   }
-  g_maps.emplace(key, m);
-  return m;
+  g_maps.emplace(key, out.map);
+  out.ok = true;
+  return out;
 }
 
-const CUtensorMap* tensor_map_2d_bf16(const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                                      uint32_t box_rows, uint32_t box_cols) {
+TensorMap tensor_map_2d_bf16(const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols) {
   uint64_t dims[2] = {cols, rows};
   uint64_t strides[1] = {ld * 2};
   uint32_t box[2] = {box_cols, box_rows};
@@ -168,6 +167,5 @@ B2_EXPORT const char* b2_last_error() { return b2::g_error_text; }
 
 B2_EXPORT void b2_clear_tensor_maps() {
   std::lock_guard<std::mutex> lock(b2::g_mu);
-  for (auto& kv : b2::g_maps) delete kv.second;
   b2::g_maps.clear();
 }

@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(MAXT) moe_norm_add_kernel(const MoeAddParams p
 }
 
 template <int BN, int FORM>
-static int launch_moe(const CUtensorMap* ta, const CUtensorMap* tb, const MoeGemmParams& p, int bound, cudaStream_t stream) {
+static int launch_moe(const TensorMap& ta, const TensorMap& tb, const MoeGemmParams& p, int bound, cudaStream_t stream) {
   using Cfg = MoeCfg<BN>;
   auto kern = moe_gemm_kernel<BN, FORM>;
   int* status = status_ptr();
@@ -800,11 +800,11 @@ static int launch_moe(const CUtensorMap* ta, const CUtensorMap* tb, const MoeGem
 
 // Gate and up [E, 2, F, K] in tiles of `cols` activation columns.
 template <int FORM>
-static int launch_glu(const CUtensorMap* ta, const void* w, const MoeGemmParams& p, int cols, int bound, cudaStream_t stream) {
+static int launch_glu(const TensorMap& ta, const void* w, const MoeGemmParams& p, int cols, int bound, cudaStream_t stream) {
   const uint64_t dims[3] = {static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.N), 2ull * p.E},
                  strides[2] = {2ull * p.K, 2ull * p.N * p.K};
   const uint32_t box[3] = {MG_BK, static_cast<uint32_t>(cols), 1};
-  const CUtensorMap* tb = tensor_map_nd_bf16(w, 3, dims, strides, box, 3);
+  const TensorMap tb = tensor_map_nd_bf16(w, 3, dims, strides, box, 3);
   if (!ta || !tb) return 2;
   if (cols == 128) return launch_moe<256, FORM>(ta, tb, p, bound, stream);
   if (cols == 64) return launch_moe<128, FORM>(ta, tb, p, bound, stream);
@@ -1014,7 +1014,7 @@ B2_EXPORT int b2_moe_down(const void* a, const void* w, const int* offsets, void
   const uint64_t dims[3] = {static_cast<uint64_t>(F), static_cast<uint64_t>(N), static_cast<uint64_t>(E)},
                  strides[2] = {2ull * F, 2ull * N * F};
   const uint32_t box[3] = {MG_BK, static_cast<uint32_t>(cols), 1};
-  const CUtensorMap *tb = tensor_map_nd_bf16(w, 3, dims, strides, box, 3), *ta = tensor_map_2d_bf16(a, P, F, F, MG_BM, MG_BK);
+  const TensorMap tb = tensor_map_nd_bf16(w, 3, dims, strides, box, 3), ta = tensor_map_2d_bf16(a, P, F, F, MG_BM, MG_BK);
   if (!ta || !tb) return 2;
   const MoeGemmParams p = {nullptr, offsets, static_cast<moe_bf16*>(out), N, P, E, N, F, GluAct{}};
   const int bound = moe_bound(P, E, MG_BM);

@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(RG_THREADS, 1) rec_gates_kernel(const __grid_c
 }
 
 template <bool OUT>
-static int launch_gates(const CUtensorMap* tu, const CUtensorMap* tw, const RecParams& p, int nchunks, cudaStream_t stream) {
+static int launch_gates(const TensorMap& tu, const TensorMap& tw, const RecParams& p, int nchunks, cudaStream_t stream) {
   auto kern = rec_gates_kernel<OUT>;
   int* status = status_ptr();
   if (!status) return 3;
@@ -606,7 +606,7 @@ B2_EXPORT int b2_gated_recurrence(const void* u, const void* w, const void* zb, 
   const RecParams p = {u, nullptr, zb, lam, y, yb, out, state, ws, nullptr, start, slot, chunks, first, C, 0, ld_y, ld_out, C, block, seq0};
   const uint64_t n = block, dims[3] = {n, n, 2ull * (C / block)}, strides[2] = {2 * n, 2 * n * n};
   const uint32_t box[3] = {64, 128, 1};
-  const CUtensorMap *tw = tensor_map_nd_bf16(w, 3, dims, strides, box, 3), *tu = tensor_map_2d_bf16(u, M, C, C, RG_CHUNK, 64);
+  const TensorMap tw = tensor_map_nd_bf16(w, 3, dims, strides, box, 3), tu = tensor_map_2d_bf16(u, M, C, C, RG_CHUNK, 64);
   if (!tw || !tu) return 2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (const int rc = launch_gates<false>(tu, tw, p, nchunks, st)) return rc;
