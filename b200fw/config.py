@@ -308,8 +308,8 @@ def apply_determinism(enabled: bool, seed: int = 0) -> None:
     """``runtime.deterministic`` (scripts/run_colocate.py:144-170 of the reference).  On: seed Python / NumPy / torch,
     ask torch for deterministic algorithms (warn only), fix cuDNN's choices, and set ``B200FW_DETERMINISTIC=1`` so the
     GEMM keeps one unit per output tile instead of split-K slices that add with float atomics.  What stays
-    order-dependent in fp32: the loss sum, the norm weight-gradient and embedding-gradient accumulations (float
-    atomics inside those kernels) - runs then agree to summation-order rounding, not bit for bit.  Off: the switches
+    order-dependent in fp32: the loss sum, the query / key norm weight-gradient and embedding-gradient accumulations
+    (float atomics inside those kernels) - runs then agree to summation-order rounding, not bit for bit.  Off: the switches
     are cleared, so a previous setting in the process or its environment does not linger."""
     import os
     import random
