@@ -185,7 +185,7 @@ class ModelRunner:
             # 100 to 4000 386 / 378, 366 / 352; but 128 of 3000 to 4000 297 / 302, 236 / 253; 256 of 512 to 1024 148 / 159,
             # 127 / 144 (three parts).
             pairs, longest = ctx.num_seqs * self.cfg.num_kv_heads, ctx.max_context_len
-            if pairs > self.num_sms and longest > 2048 and 2 * longest * ctx.num_seqs > 3 * ctx.total_k:
+            if pairs > self.num_sms and longest > 2048 and 0 < 3 * ctx.total_k < 2 * longest * ctx.num_seqs:
                 part = (-(-longest // 4) + 63) // 64 * 64
                 return part, -(-longest // part)
         return 0, 1

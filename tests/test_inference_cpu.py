@@ -50,7 +50,9 @@ def test_balanced_splits_are_for_unequal_contexts(lens, kv_heads, plan):
     r = NS(enable_partitioned=False, balance_splits=True, num_sms=148, cfg=NS(num_heads=8 * kv_heads, num_kv_heads=kv_heads))
     ctx = NS(num_seqs=len(lens), max_context_len=max(lens), total_k=sum(lens))
     assert ModelRunner._split_plan(r, ctx) == plan
-    r.balance_splits = False
+    ctx.total_k = 0                  # a caller's own context that does not say how long its sequences are
+    assert ModelRunner._split_plan(r, ctx) == (0, 1)
+    r.balance_splits, ctx.total_k = False, sum(lens)
     assert ModelRunner._split_plan(r, ctx) == (0, 1)
 
 
