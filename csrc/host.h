@@ -52,8 +52,8 @@ inline int num_sms() {
   return n[dev];
 }
 
-// B200FW_BATCH_INVARIANT=1: a row's sums are taken in one order, however many rows or sequences there are beside it: no products
-// or contexts dealt to a cluster, which the dispatch does by how many there are.
+// B200FW_BATCH_INVARIANT=1: products and paged decode attention take a row's sums in one order, however many rows or sequences
+// there are beside it: nothing dealt to a cluster or cut into slices, which the dispatch does by how many there are.
 inline bool batch_invariant() {
   static const bool on = [] {
     const char* e = std::getenv("B200FW_BATCH_INVARIANT");

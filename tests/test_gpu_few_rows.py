@@ -299,6 +299,12 @@ for n, k in ((1024, 3072), (4096, 1024), (2560, 9728)):
     alone = ops.linear(x[:1], w, r[:1])
     for m in (2, 64, 130, 1100):
         assert torch.equal(ops.linear(x[:m], w, r[:m])[:1], alone), (n, k, m)
+x, w, first = rnd(1100, 3072), rnd(4096, 3072), rnd(1100, 4096).float()      # 32-bit outputs, added to what is there or not
+for add in (False, True):
+    run = lambda m: ops.gemm(x[:m], w, out=first[:m].clone(), accumulate=add)
+    alone = run(1)
+    for m in (2, 64, 130, 1100):
+        assert torch.equal(run(m)[:1], alone), (add, m)
 B, Hq, Hkv, n = 300, 16, 8, 700
 pages = -(-n // 16)
 kc, vc, q = rnd(4 * pages, 16, Hkv, 128), rnd(4 * pages, 16, Hkv, 128), rnd(B, Hq * 128)
